@@ -261,6 +261,9 @@ struct bpgb_plan_s {
     Factorization fz{};
     bpgb_pair *d_pairs = nullptr;
     FastPlan *fast = nullptr;
+    ExactFilter filter{};  // EXACT
+    uint32_t splits = 1;         // EXACT: CTAs per voxel tile
+    void *d_partial = nullptr;   // EXACT: their partial volumes
     cudaStream_t last_stream = nullptr;
 };
 
@@ -371,6 +374,18 @@ int bpgb_plan_create(bpgb_plan *plan, const bpgb_pair *host_pairs, uint64_t num_
         }
     }
     p->algo = algo;
+    if (algo == BPGB_ALGO_EXACT) {
+        p->filter = exact_filter(host_pairs, num_pairs, p->vol, p->bp);
+        p->splits = exact_splits(p->vol, num_pairs, sms);
+        if (p->splits > 1) {
+            const size_t esz = o.h_dtype == BPGB_DTYPE_C64 ? 8 : 4;
+            if (cudaMalloc(&p->d_partial, p->splits * p->vol.count() * esz) != cudaSuccess) {
+                cudaGetLastError();  // no room for partial volumes: one CTA per tile
+                p->d_partial = nullptr;
+                p->splits = 1;
+            }
+        }
+    }
     *plan = p;
     return BPGB_OK;
 }
@@ -390,7 +405,7 @@ int bpgb_plan_execute(bpgb_plan plan, const void *d_H, void *d_volume, void *str
     if (plan->algo == BPGB_ALGO_FAST) return fast_plan_execute(plan->fast, d_H, d_volume, s);
     const uint64_t pitch = plan->opt.h_pitch ? plan->opt.h_pitch : plan->bp.T;
     int st = launch_exact(d_H, cplx, pitch, plan->d_pairs, plan->P, plan->vol, plan->bp,
-                          d_volume, s);
+                          plan->filter, plan->splits, plan->d_partial, d_volume, s);
     if (st) return st;
     if (plan->opt.h_scale != 1.0f && plan->opt.h_scale != 0.0f)
         return set_error(BPGB_ERR_UNSUPPORTED, "h_scale applies to the FAST path only");
@@ -464,11 +479,14 @@ int bpgb_plan_get_info(bpgb_plan plan, bpgb_plan_info *info) {
     info->tile[0] = 4;
     info->tile[1] = 8;
     info->tile[2] = 8;
-    info->pair_splits = 1;
-    info->grid = (uint32_t)(((plan->vol.n[0] + 3) / 4) * ((plan->vol.n[1] + 7) / 8) *
+    info->pair_splits = plan->splits;
+    info->grid = plan->splits * (uint32_t)(((plan->vol.n[0] + 3) / 4) * ((plan->vol.n[1] + 7) / 8) *
                             ((plan->vol.n[2] + 7) / 8));
-    info->threads = 256;
-    info->scratch_bytes = plan->P * sizeof(bpgb_pair);
+    info->threads = 64;
+    info->scratch_bytes = plan->P * sizeof(bpgb_pair) +
+                          (plan->splits > 1 ? plan->splits * plan->vol.count() *
+                                                  (plan->opt.h_dtype == BPGB_DTYPE_C64 ? 8 : 4)
+                                            : 0);
     return BPGB_OK;
 }
 
@@ -514,6 +532,7 @@ int bpgb_plan_destroy(bpgb_plan plan) {
     if (!plan) return BPGB_OK;
     if (plan->fast) fast_plan_free(plan->fast);
     if (plan->d_pairs) cudaFree(plan->d_pairs);
+    if (plan->d_partial) cudaFree(plan->d_partial);
     delete plan;
     return BPGB_OK;
 }
