@@ -1714,6 +1714,29 @@ int fast_args(FastArgs &a, const FastConfig &cfg, const Volume &vol, const doubl
     return BPGB_OK;
 }
 
+// Pair splits of a launch of `groups` CTAs per split over `items` work items each: the count,
+// up to six rounds of resident CTAs, whose busiest SM finishes first.  An SM takes n CTAs,
+// `occ` at a time; a last round of r < occ CTAs, with fewer warps to hide latency, lasts like
+// r + 0.3 (occ - r) of them in a full round; a CTA's start-up costs about a quarter of an
+// item.  Those two constants were fitted to sixteen captures (8 to 720 tiles, every scan and
+// row type) timed at every split count: the rule's choice is 1.0% from the best on average
+// (at most 10%), where filling two rounds regardless of the remainder was 10% (32%): 64^3
+// voxels, 4,096 pairs, 8 -> 7 splits 322 -> 318 us; 34 x 62 x 14 voxels 39 -> 19 splits 36 ->
+// 27 us; lasers x SPADs at 32^3 38 -> 19 splits 453 -> 451 us.
+uint64_t auto_splits(uint64_t groups, uint64_t items, uint32_t sms, int occ) {
+    const uint64_t rounds = (6ull * sms * occ + groups - 1) / groups;
+    const uint64_t most = std::min<uint64_t>(items, std::max<uint64_t>(1, rounds));
+    uint64_t best = 1;
+    double best_cost = INFINITY;
+    for (uint64_t s = 1; s <= most; s++) {
+        const uint64_t n = (groups * s + sms - 1) / sms, r = n % occ;
+        const double units = (double)(n - r) + (r ? r + 0.3 * (occ - r) : 0.0);
+        const double cost = units * ((double)items / (double)s + 0.25);
+        if (cost < 0.995 * best_cost) best = s, best_cost = cost;
+    }
+    return best;
+}
+
 uint32_t fast_threads(const FastConfig &cfg) { return 32 * (1 + cfg.cta_consumer_warps()); }
 uint32_t fast_smem(const FastArgs &a) { return a.stages * a.stage_bytes + 128; }
 
@@ -1862,11 +1885,8 @@ int fast_plan_build(FastPlan **out, const bpgb_pair *d_pairs, uint64_t P,
     const uint64_t ntiles = (uint64_t)a.tiles[0] * a.tiles[1] * a.tiles[2];
     const uint64_t ngroups = (ntiles + a.groups - 1) / a.groups;  // CTAs per pair split
     const uint64_t items = fast_items(a);
-    uint64_t splits = opt.pair_splits > 0 ? (uint64_t)opt.pair_splits : 1;
-    if (opt.pair_splits <= 0) {
-        const uint64_t want = 2ull * sm_count * occ;  // two waves of resident CTAs
-        if (ngroups < want) splits = (want + ngroups - 1) / ngroups;
-    }
+    uint64_t splits = opt.pair_splits > 0 ? (uint64_t)opt.pair_splits
+                                          : auto_splits(ngroups, items, (uint32_t)sm_count, occ);
     splits = std::max<uint64_t>(1, std::min<uint64_t>(splits, items));
     if (ngroups * splits >= (1ull << 31)) {
         fast_plan_free(fp);
@@ -2914,9 +2934,7 @@ extern "C" int bpgb_backproject_noalloc(const float *d_H, uint32_t T, uint32_t h
     if (occ < 1) return set_error(BPGB_ERR_UNSUPPORTED, "fast kernel does not fit on an SM");
     const uint64_t ntiles = (uint64_t)a.tiles[0] * a.tiles[1] * a.tiles[2];
     const uint64_t items = a.L * a.nchunks;
-    uint64_t splits = 1;
-    const uint64_t want = 2ull * sms * occ;
-    if (ntiles < want) splits = (want + ntiles - 1) / ntiles;
+    uint64_t splits = auto_splits(ntiles, items, (uint32_t)sms, occ);
     // partial sums must fit next to the tables: fewer splits, never an error
     const uint64_t part_off = (kNoAllocDiagBytes + tab_bytes + 255) / 256 * 256;
     const uint64_t part_room = kNoAllocScratchBytes - std::min<uint64_t>(kNoAllocScratchBytes, part_off);
