@@ -3,9 +3,18 @@
 // out[r, t] = sum_{k=0}^{K-1} H[r, t + k - K/2] * (cos_k, sin_k) over read indices in
 // (0, T) (index 0 is excluded, :468).  The sum runs in tap order with a separate FP32
 // multiply and add per tap, as the reference's loop does, so the result matches a CPU
-// evaluation of that loop bit for bit.  Each CTA stages one row segment plus its halo
-// in shared memory (zeros outside (0, T), which reproduces the index test), and each
-// thread produces 8 outputs strided by the block size (conflict-free shared reads).
+// evaluation of that loop bit for bit.
+//
+// Bound: the FP32 pipe and issue, two multiplies and two adds per output and tap (fused or
+// reordered sums would change bits).  A thread owns 8 consecutive outputs, so each row value,
+// loaded once into a register, serves the 8 outputs as the taps slide over it: 33 issue slots
+// per tap and 8 outputs, where strided outputs, each with its own load, took 41.  Each CTA
+// stages one row segment plus its halo in shared memory (zeros outside (0, T), which
+// reproduces the index test), groups of 8 values 48 bytes apart so that the lanes' 16-byte
+// loads hit distinct banks.  Measured on 16,384 rows of 4,096 bins and 503 taps: 4.79 ms
+// before, 3.94 ms now (3.4 ms at 128 FP32 results per SM and clock).  Packed FP32x2 sums
+// measured 4.12 ms; packed products are fused with packed sums whatever their rounding
+// modifiers, which changes bits.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -19,45 +28,108 @@
 namespace bpgb {
 namespace {
 
-constexpr int kThreads = 128;
-constexpr int kPerThread = 8;
-constexpr int kSeg = kThreads * kPerThread;
+constexpr int kPer = 8;              // consecutive outputs per thread
+constexpr int kMaxThreads = 128;
+constexpr int kSeg = kMaxThreads * kPer;
+constexpr int kTapBlock = 512;       // taps staged at a time, a multiple of kPer
+constexpr int kGroupWords = kPer + 4;  // a staged group of 8 values, padded
 
-__global__ void __launch_bounds__(kThreads)
+// Threads of a CTA (8 outputs each) and segments of a row: T split evenly over as few
+// segments as kSeg allows.
+struct PulseShape {
+    uint32_t nseg, threads;
+    uint32_t smem;
+};
+
+PulseShape pulse_shape(uint32_t T, int K) {
+    PulseShape p;
+    p.nseg = (T + kSeg - 1) / kSeg;
+    const uint32_t per = (T + p.nseg - 1) / p.nseg;
+    p.threads = ((per + kPer - 1) / kPer + 31) / 32 * 32;
+    const int kt = std::min(K, kTapBlock);
+    const uint32_t groups = p.threads + (kt + kPer - 1) / kPer + 2;
+    p.smem = (groups * kGroupWords + 2 * (kt + 1)) * sizeof(float);
+    return p;
+}
+
+// acc += x * c, products and sums rounded separately.
+__device__ __forceinline__ void mul_add(float2 &acc, float x, float2 c) {
+    acc.x = __fadd_rn(acc.x, __fmul_rn(x, c.x));
+    acc.y = __fadd_rn(acc.y, __fmul_rn(x, c.y));
+}
+
+__global__ void __launch_bounds__(kMaxThreads)
     phasor_pulse_kernel(const float *__restrict__ H, uint32_t T, uint32_t in_pitch,
                         const float2 *__restrict__ taps, int K, float2 *__restrict__ out,
-                        uint32_t out_pitch, uint32_t nseg) {
-    extern __shared__ float sm[];
-    float *seg = sm;                                         // kSeg + K entries
-    float2 *tp = reinterpret_cast<float2 *>(sm + ((kSeg + K + 1) & ~1));
+                        uint32_t out_pitch, uint32_t nseg, int vec) {
+    extern __shared__ __align__(16) float sm[];
+    const int groups = blockDim.x + (min(K, kTapBlock) + kPer - 1) / kPer + 2;
+    float4 *tp4 = reinterpret_cast<float4 *>(sm + (size_t)groups * kGroupWords);
+    float2 *tp = reinterpret_cast<float2 *>(tp4);
     const uint64_t r = blockIdx.x / nseg;
     const uint32_t sg = blockIdx.x % nseg;
-    const int64_t t_begin = (int64_t)sg * kSeg;
-    const int half = K / 2;
+    const int64_t t_begin = (int64_t)sg * blockDim.x * kPer;
     const float *row = H + r * in_pitch;
-    for (int i = threadIdx.x; i < kSeg + K; i += kThreads) {
-        const int64_t ri = t_begin - half + i;
-        seg[i] = (ri > 0 && ri < (int64_t)T) ? row[ri] : 0.0f;
-    }
-    for (int k = threadIdx.x; k < K; k += kThreads) tp[k] = taps[k];
-    __syncthreads();
-    float re[kPerThread], im[kPerThread];
+    auto load_group = [&](int g, float (&x)[kPer]) {
+        const float4 *p = reinterpret_cast<const float4 *>(sm + (size_t)g * kGroupWords);
+        const float4 a = p[0], b = p[1];
+        x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+        x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    };
+    float2 acc[kPer];
 #pragma unroll
-    for (int j = 0; j < kPerThread; j++) re[j] = im[j] = 0.0f;
-    for (int k = 0; k < K; k++) {
-        const float2 c = tp[k];
+    for (int j = 0; j < kPer; j++) acc[j] = make_float2(0.0f, 0.0f);
+    for (int k0 = 0; k0 < K; k0 += kTapBlock) {
+        const int kt = min(K - k0, kTapBlock);
+        if (k0 > 0) __syncthreads();
+        for (int i = threadIdx.x; i < groups * kPer; i += blockDim.x) {
+            const int64_t ri = t_begin - K / 2 + k0 + i;
+            const float v = (ri > 0 && ri < (int64_t)T) ? row[ri] : 0.0f;
+            sm[(i / kPer) * kGroupWords + i % kPer] = v;
+        }
+        for (int k = threadIdx.x; k < kt; k += blockDim.x) tp[k] = taps[k0 + k];
+        __syncthreads();
+        float x0[kPer], x1[kPer];
+        load_group(threadIdx.x, x0);
+        const int full = kt / kPer;
+#pragma unroll 2
+        for (int kb = 0; kb < full; kb++) {
+            load_group(threadIdx.x + kb + 1, x1);
 #pragma unroll
-        for (int j = 0; j < kPerThread; j++) {
-            const float x = seg[threadIdx.x + j * kThreads + k];
-            re[j] = __fadd_rn(re[j], __fmul_rn(x, c.x));
-            im[j] = __fadd_rn(im[j], __fmul_rn(x, c.y));
+            for (int u = 0; u < kPer; u += 2) {
+                const float4 c = tp4[(kb * kPer + u) / 2];
+#pragma unroll
+                for (int j = 0; j < kPer; j++)
+                    mul_add(acc[j], u + j < kPer ? x0[u + j] : x1[u + j - kPer],
+                            make_float2(c.x, c.y));
+#pragma unroll
+                for (int j = 0; j < kPer; j++)
+                    mul_add(acc[j], u + 1 + j < kPer ? x0[u + 1 + j] : x1[u + 1 + j - kPer],
+                            make_float2(c.z, c.w));
+            }
+#pragma unroll
+            for (int j = 0; j < kPer; j++) x0[j] = x1[j];
+        }
+        for (int k = full * kPer; k < kt; k++) {  // the last K mod 8 taps
+            const float2 c = tp[k];
+#pragma unroll
+            for (int j = 0; j < kPer; j++) {
+                const int i = threadIdx.x * kPer + k + j;
+                mul_add(acc[j], sm[(i / kPer) * kGroupWords + i % kPer], c);
+            }
         }
     }
-    float2 *orow = out + r * out_pitch;
+    const int64_t t = t_begin + threadIdx.x * kPer;
+    float2 *o = out + r * out_pitch + t;
+    if (vec && t + kPer <= (int64_t)T) {
 #pragma unroll
-    for (int j = 0; j < kPerThread; j++) {
-        const int64_t t = t_begin + threadIdx.x + j * kThreads;
-        if (t < (int64_t)T) orow[t] = make_float2(re[j], im[j]);
+        for (int j = 0; j < kPer / 2; j++)
+            reinterpret_cast<float4 *>(o)[j] =
+                make_float4(acc[2 * j].x, acc[2 * j].y, acc[2 * j + 1].x, acc[2 * j + 1].y);
+    } else {
+#pragma unroll
+        for (int j = 0; j < kPer; j++)
+            if (t + j < (int64_t)T) o[j] = acc[j];
     }
 }
 
@@ -104,16 +176,17 @@ int launch_phasor_pulse(const float *d_H, uint64_t rows, uint32_t T, uint32_t in
         BPGB_CUDA_TRY(cudaMemset2DAsync(d_out, (size_t)out_pitch * 8, 0, (size_t)T * 8, rows, stream));
         return BPGB_OK;
     }
-    const uint32_t nseg = (T + kSeg - 1) / kSeg;
-    const size_t smem = (size_t)(((kSeg + K + 1) & ~1) + 2 * K) * sizeof(float);
-    if (smem > 200 * 1024) return set_error(BPGB_ERR_UNSUPPORTED, "phasor pulse too long for shared memory");
-    const uint64_t blocks = rows * nseg;
+    const PulseShape p = pulse_shape(T, K);
+    if ((size_t)(((kSeg + K + 1) & ~1) + 2 * K) * sizeof(float) > 200 * 1024) return set_error(BPGB_ERR_UNSUPPORTED, "phasor pulse too long");
+    const uint64_t blocks = rows * p.nseg;
     if (blocks >= (1ull << 31)) return set_error(BPGB_ERR_UNSUPPORTED, "too many rows for one launch");
     const float2 *d_taps = nullptr;
     if (int st = device_taps(h_taps, K, &d_taps)) return st;
-    if (int rs = reserve_dynamic_smem((const void *)phasor_pulse_kernel, (uint32_t)smem)) return rs;
-    phasor_pulse_kernel<<<(unsigned)blocks, kThreads, smem, stream>>>(
-        d_H, T, in_pitch, d_taps, K, reinterpret_cast<float2 *>(d_out), out_pitch, nseg);
+    if (int rs = reserve_dynamic_smem((const void *)phasor_pulse_kernel, p.smem)) return rs;
+    // 16-byte stores where every row's outputs are 16-byte aligned
+    const int vec = ((uintptr_t)d_out % 16 == 0 && out_pitch % 2 == 0) ? 1 : 0;
+    phasor_pulse_kernel<<<(unsigned)blocks, p.threads, p.smem, stream>>>(
+        d_H, T, in_pitch, d_taps, K, reinterpret_cast<float2 *>(d_out), out_pitch, p.nseg, vec);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;
