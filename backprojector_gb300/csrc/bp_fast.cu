@@ -1250,65 +1250,165 @@ __global__ void __launch_bounds__(288, kFactCtas)
     pipeline_drain(a.stages, step, full_bar, diag, a.spin_limit);
 }
 
-// out[v] = scale * sum_s partial[s][v], in split order (optionally Kahan).
-template <bool COMPLEX, bool KAHAN>
-__global__ void reduce_splits_kernel(const float *__restrict__ partial, float *__restrict__ out,
-                                     uint64_t nvox, uint32_t splits, float scale) {
-    constexpr int C = COMPLEX ? 2 : 1;
-    const uint64_t n = nvox * C;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        float s = 0.0f, c = 0.0f;
-        for (uint32_t k = 0; k < splits; k++) {
-            const float x = partial[(uint64_t)k * n + i];
-            if (KAHAN)
-                kahan_add(s, c, x);
-            else
-                s += x;
-        }
-        if (KAHAN) s -= c;
-        out[i] = s * scale;
-    }
+// ---- partial sums of pair splits -------------------------------------------------------
+// A voxel's sum over its splits: sums of kSegment consecutive splits, each in split order,
+// added in order (Kahan-compensated sums: one chain over all splits).  Both reductions below
+// form it the same way, so a tile-list voxel equals the full-volume one bit for bit.
+constexpr uint32_t kSegment = 8;
+
+// Splits [k0, min(k0 + kSegment, splits)) of 4 floats; load(k) is split k's value.
+template <typename Load>
+__device__ __forceinline__ float4 segment_sum(uint32_t k0, uint32_t splits, Load &&load) {
+    float4 v[kSegment];  // all loads in flight before the first add
+#pragma unroll
+    for (uint32_t k = 0; k < kSegment; k++)
+        v[k] = k0 + k < splits ? load(k0 + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 s = v[0];
+#pragma unroll
+    for (uint32_t k = 1; k < kSegment; k++)
+        if (k0 + k < splits) s.x += v[k].x, s.y += v[k].y, s.z += v[k].z, s.w += v[k].w;
+    return s;
 }
 
-// Tile-list form of reduce_splits_kernel: slot s < *count holds tile list[s]; the
-// partial sums of its splits (slot-major, then split, then tile-local voxel) are added in split order
-// with the same arithmetic, so a voxel equals the full-volume reduction bit for bit.
+template <bool KAHAN, typename Load>
+__device__ __forceinline__ float4 splits_sum(uint32_t splits, Load &&load) {
+    if (KAHAN) {
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = s;
+        for (uint32_t k = 0; k < splits; k++) {
+            const float4 x = load(k);
+            kahan_add(s.x, c.x, x.x);
+            kahan_add(s.y, c.y, x.y);
+            kahan_add(s.z, c.z, x.z);
+            kahan_add(s.w, c.w, x.w);
+        }
+        return make_float4(s.x - c.x, s.y - c.y, s.z - c.z, s.w - c.w);
+    }
+    float4 s = segment_sum(0, splits, load);
+    for (uint32_t k = kSegment; k < splits; k += kSegment) {
+        const float4 t = segment_sum(k, splits, load);
+        s.x += t.x, s.y += t.y, s.z += t.z, s.w += t.w;
+    }
+    return s;
+}
+
+// n floats at p + i, fewer than 4 at the end; `vec`: p is 16-byte aligned
+__device__ __forceinline__ float4 load4(const float *p, uint64_t i, uint64_t n, bool vec) {
+    if (vec && i + 4 <= n) return *reinterpret_cast<const float4 *>(p + i);
+    float4 v = make_float4(p[i], 0.0f, 0.0f, 0.0f);
+    if (i + 1 < n) v.y = p[i + 1];
+    if (i + 2 < n) v.z = p[i + 2];
+    if (i + 3 < n) v.w = p[i + 3];
+    return v;
+}
+__device__ __forceinline__ void store4(float *p, uint64_t i, uint64_t n, bool vec, float4 v) {
+    if (vec && i + 4 <= n) {
+        *reinterpret_cast<float4 *>(p + i) = v;
+        return;
+    }
+    p[i] = v.x;
+    if (i + 1 < n) p[i + 1] = v.y;
+    if (i + 2 < n) p[i + 2] = v.z;
+    if (i + 3 < n) p[i + 3] = v.w;
+}
+__device__ __forceinline__ float4 scaled(float4 v, float f) {
+    return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+}
+
+// out[i] = scale * (sum of partial[s][i] over the splits), i < n floats.  A block takes
+// 256 groups of 4 floats, one per thread; with more than kSegment splits and too few groups
+// for a GPU full of threads (`rows`), kReduceX groups, whose segments are summed by the other
+// rows of threads and added by row 0 in order.  Latency bounds it (each float is read once):
+// 4,096 voxels x 64 splits 8.7 -> 3.6 us, 262,144 voxels x 7 splits 4.6 -> 3.9 us against one
+// thread and one chain of loads per voxel.
+constexpr uint32_t kReduceX = 32, kReduceY = 8;
+template <bool KAHAN>
+__global__ void __launch_bounds__(kReduceX *kReduceY)
+    reduce_splits_kernel(const float *__restrict__ partial, float *__restrict__ out, uint64_t n,
+                         uint32_t splits, float scale, int vec, int rows) {
+    const uint64_t quads = (n + 3) / 4;
+    const bool vp = vec && n % 4 == 0;  // every split's block is 16-byte aligned
+    if (KAHAN || !rows) {
+        const uint64_t i = 4 * ((uint64_t)blockIdx.x * (kReduceX * kReduceY) + threadIdx.y * kReduceX +
+                                threadIdx.x);
+        if (i >= n) return;
+        auto load = [&](uint32_t k) { return load4(partial + k * n, i, n, vp); };
+        store4(out, i, n, vec, scaled(splits_sum<KAHAN>(splits, load), scale));
+        return;
+    }
+    __shared__ float4 seg[kReduceY][kReduceX];
+    const uint64_t q = (uint64_t)blockIdx.x * kReduceX + threadIdx.x, i = 4 * q;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (uint32_t k0 = 0; k0 < splits; k0 += kReduceY * kSegment) {
+        const uint32_t k = k0 + threadIdx.y * kSegment;
+        if (q < quads && k < splits)
+            seg[threadIdx.y][threadIdx.x] = segment_sum(
+                k, splits, [&](uint32_t s) { return load4(partial + s * n, i, n, vp); });
+        __syncthreads();
+        if (threadIdx.y == 0) {
+            for (uint32_t y = 0; y < kReduceY && k0 + y * kSegment < splits; y++) {
+                const float4 t = seg[y][threadIdx.x];
+                if (k0 + y == 0)
+                    sum = t;
+                else
+                    sum.x += t.x, sum.y += t.y, sum.z += t.z, sum.w += t.w;
+            }
+        }
+        __syncthreads();
+    }
+    if (threadIdx.y == 0 && q < quads) store4(out, i, n, vec, scaled(sum, scale));
+}
+
+// Queues reduce_splits_kernel over n floats.
+void launch_reduce_splits(const float *partial, float *out, uint64_t n, uint32_t splits, float scale,
+                          bool kahan, cudaStream_t s) {
+    const uint64_t quads = (n + 3) / 4;
+    // below 64 K groups a thread per group leaves most of the 300 K resident threads idle
+    // (106,750 groups x 13 splits: 9.0 us a thread per group, 11.5 us in rows)
+    const int rows = !kahan && splits > kSegment && quads < 65536;
+    const uint32_t per = rows ? kReduceX : kReduceX * kReduceY;
+    const unsigned blocks = (unsigned)((quads + per - 1) / per);
+    const int vec = (uintptr_t)partial % 16 == 0 && (uintptr_t)out % 16 == 0;
+    const dim3 threads(kReduceX, kReduceY);
+    if (kahan)
+        reduce_splits_kernel<true><<<blocks, threads, 0, s>>>(partial, out, n, splits, scale, vec, rows);
+    else
+        reduce_splits_kernel<false><<<blocks, threads, 0, s>>>(partial, out, n, splits, scale, vec, rows);
+    count_launches(1);
+}
+
+// Tile-list form: slot s < *count holds tile list[s]; the partial sums of its splits (slot-
+// major, then split, then tile-local voxel) are added as above.  One slot per CTA at a time,
+// 4 floats of a z line per thread.  1,050 8^3 tiles x 8 splits: 11.8 -> 8.0 us against one
+// voxel and several 64-bit divisions per thread.
 template <bool COMPLEX, bool KAHAN>
-__global__ void reduce_tiles_kernel(const float *__restrict__ partial,
-                                    const uint32_t *__restrict__ list,
-                                    const uint32_t *__restrict__ count, uint32_t max_tiles,
-                                    const FastArgs a, float *__restrict__ out) {
-    constexpr int C = COMPLEX ? 2 : 1;
-    const uint64_t tvox = (uint64_t)a.tdim[0] * a.tdim[1] * a.tdim[2];
-    const uint64_t n = (uint64_t)max_tiles * tvox * C;
-    const uint32_t cnt = *count;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t slot = i / (tvox * C);
-        if (slot >= cnt) break;
-        const uint64_t r = i - slot * tvox * C;
-        const uint64_t local = r / C;
-        const uint32_t c = (uint32_t)(r - local * C);
+__global__ void __launch_bounds__(128)
+    reduce_tiles_kernel(const float *__restrict__ partial, const uint32_t *__restrict__ list,
+                        const uint32_t *__restrict__ count, uint32_t max_tiles, const FastArgs a,
+                        float *__restrict__ out, int vec, const float *d_absmax, float target) {
+    const float factor = scale_of(1.0f, d_absmax, target);
+    constexpr uint32_t C = COMPLEX ? 2 : 1;
+    const uint32_t tz4 = a.tdim[2] * C / 4;  // tiles are a multiple of 4 voxels along z
+    const uint32_t quads = a.tdim[0] * a.tdim[1] * tz4;
+    const uint64_t tfloats = 4ull * quads, line = (uint64_t)a.n[2] * C;
+    const uint32_t slots = min(*count, max_tiles);
+    for (uint32_t slot = blockIdx.x; slot < slots; slot += gridDim.x) {
         const uint32_t tile = list[slot];
         if (tile >= (uint64_t)a.tiles[0] * a.tiles[1] * a.tiles[2]) continue;  // skipped entry
-        const uint32_t tz = tile % a.tiles[2], tx = (tile / a.tiles[2]) % a.tiles[0],
-                       ty = tile / (a.tiles[2] * a.tiles[0]);
-        const uint32_t lz = (uint32_t)(local % a.tdim[2]),
-                       ly = (uint32_t)((local / a.tdim[2]) % a.tdim[1]),
-                       lx = (uint32_t)(local / ((uint64_t)a.tdim[2] * a.tdim[1]));
-        const uint32_t x = tx * a.tdim[0] + lx, y = ty * a.tdim[1] + ly, z = tz * a.tdim[2] + lz;
-        if (x >= a.n[0] || y >= a.n[1] || z >= a.n[2]) continue;
-        float s = 0.0f, cmp = 0.0f;
-        for (uint32_t k = 0; k < a.splits; k++) {
-            const float v = partial[((slot * a.splits + k) * tvox + local) * C + c];
-            if (KAHAN)
-                kahan_add(s, cmp, v);
-            else
-                s += v;
+        TileGeo g;
+        tile_of_block(a, tile, g);
+        const float *p = partial + (uint64_t)slot * a.splits * tfloats;
+        for (uint32_t q = threadIdx.x; q < quads; q += 128) {
+            const uint32_t z4 = q % tz4, xy = q / tz4;
+            const uint32_t x = g.org[0] + xy / a.tdim[1], y = g.org[1] + xy % a.tdim[1];
+            const uint64_t z = (uint64_t)g.org[2] * C + 4 * z4;  // in floats
+            if (x >= a.n[0] || y >= a.n[1] || z >= line) continue;
+            auto load = [&](uint32_t k) {
+                return *reinterpret_cast<const float4 *>(p + k * tfloats + 4ull * q);
+            };
+            float4 v = scaled(splits_sum<KAHAN>(a.splits, load), a.out_scale);
+            if (d_absmax) v = scaled(v, factor);
+            store4(out + ((uint64_t)x * a.n[1] + y) * line, z, line, vec, v);
         }
-        if (KAHAN) s -= cmp;
-        out[(((uint64_t)x * a.n[1] + y) * a.n[2] + z) * C + c] = s * a.out_scale;
     }
 }
 
@@ -1967,35 +2067,22 @@ int fast_plan_execute(FastPlan *fp, const void *d_H, void *d_out, cudaStream_t s
     count_launches(1);
     if (a.splits > 1) {
         const bool cplx = fp->dtype == BPGB_DTYPE_C64 || fp->dtype == BPGB_DTYPE_C32;
-        const uint64_t n = a.nvox * (cplx ? 2 : 1);
-        const unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, 152ull * 8);
-        if (cplx) {
-            if (fp->kahan)
-                reduce_splits_kernel<true, true><<<blocks, 256, 0, stream>>>(
-                    fp->d_partial, (float *)d_out, a.nvox, a.splits, a.out_scale);
-            else
-                reduce_splits_kernel<true, false><<<blocks, 256, 0, stream>>>(
-                    fp->d_partial, (float *)d_out, a.nvox, a.splits, a.out_scale);
-        } else {
-            if (fp->kahan)
-                reduce_splits_kernel<false, true><<<blocks, 256, 0, stream>>>(
-                    fp->d_partial, (float *)d_out, a.nvox, a.splits, a.out_scale);
-            else
-                reduce_splits_kernel<false, false><<<blocks, 256, 0, stream>>>(
-                    fp->d_partial, (float *)d_out, a.nvox, a.splits, a.out_scale);
-        }
-        count_launches(1);
+        launch_reduce_splits(fp->d_partial, (float *)d_out, a.nvox * (cplx ? 2 : 1), a.splits,
+                             a.out_scale, fp->kahan, stream);
         BPGB_CUDA_TRY(cudaGetLastError());
     }
     return BPGB_OK;
 }
 
 int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const uint32_t *d_list,
-                            const uint32_t *d_count, uint32_t max_tiles, cudaStream_t stream) {
+                            const uint32_t *d_count, uint32_t max_tiles, cudaStream_t stream,
+                            const float *d_absmax, float target) {
     const FastArgs &a0 = fp->a;
     const uint64_t ntiles = (uint64_t)a0.tiles[0] * a0.tiles[1] * a0.tiles[2];
     if (!d_list || !d_count) return set_error(BPGB_ERR_INVALID_ARGUMENT, "null tile list");
     if (max_tiles == 0) return BPGB_OK;
+    if (d_absmax && a0.splits == 1)
+        return set_error(BPGB_ERR_UNSUPPORTED, "unsplit tile lists store unscaled voxels");
     const uint64_t slot_groups = ((uint64_t)max_tiles + a0.groups - 1) / a0.groups;
     if (slot_groups * a0.splits >= (1ull << 31))
         return set_error(BPGB_ERR_UNSUPPORTED, "tile list x pair splits too large for one grid");
@@ -2012,29 +2099,26 @@ int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const ui
     a.tile_local = a.splits > 1 ? 1 : 0;
     const float4 *spads = fp->d_tables;
     const float4 *lasers = fp->d_tables + a.S;
-    void *target = a.splits > 1 ? (void *)fp->d_partial : d_out;
+    void *dst = a.splits > 1 ? (void *)fp->d_partial : d_out;
     void *kern = plan_kernel(fp);
-    void *args[] = {(void *)&map, (void *)&spads, (void *)&lasers, (void *)&target,
+    void *args[] = {(void *)&map, (void *)&spads, (void *)&lasers, (void *)&dst,
                     (void *)&fp->d_diag, (void *)&a};
     BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3((uint32_t)(slot_groups * a.splits)),
                                    dim3(fp->threads), args, fp->smem, stream));
     count_launches(1);
     if (a.splits > 1) {
         const bool cplx = fp->dtype == BPGB_DTYPE_C64 || fp->dtype == BPGB_DTYPE_C32;
-        const uint64_t n = (uint64_t)max_tiles * a.tdim[0] * a.tdim[1] * a.tdim[2] * (cplx ? 2 : 1);
-        const unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, 152ull * 8);
+        const unsigned blocks = std::min<unsigned>(max_tiles, 152u * 16);
         float *o = (float *)d_out;
-        if (cplx) {
-            if (fp->kahan)
-                reduce_tiles_kernel<true, true><<<blocks, 256, 0, stream>>>(fp->d_partial, d_list, d_count, max_tiles, a, o);
-            else
-                reduce_tiles_kernel<true, false><<<blocks, 256, 0, stream>>>(fp->d_partial, d_list, d_count, max_tiles, a, o);
-        } else {
-            if (fp->kahan)
-                reduce_tiles_kernel<false, true><<<blocks, 256, 0, stream>>>(fp->d_partial, d_list, d_count, max_tiles, a, o);
-            else
-                reduce_tiles_kernel<false, false><<<blocks, 256, 0, stream>>>(fp->d_partial, d_list, d_count, max_tiles, a, o);
-        }
+        const int vec = (uintptr_t)d_out % 16 == 0 && (a.n[2] * (cplx ? 2 : 1)) % 4 == 0;
+        auto run = [&](auto kernel) {
+            kernel<<<blocks, 128, 0, stream>>>(fp->d_partial, d_list, d_count, max_tiles, a, o, vec,
+                                                  d_absmax, target);
+        };
+        if (cplx)
+            fp->kahan ? run(reduce_tiles_kernel<true, true>) : run(reduce_tiles_kernel<true, false>);
+        else
+            fp->kahan ? run(reduce_tiles_kernel<false, true>) : run(reduce_tiles_kernel<false, false>);
         count_launches(1);
         BPGB_CUDA_TRY(cudaGetLastError());
     }
@@ -2439,10 +2523,8 @@ int batch_execute(BatchPlan *b, const void *d_H, float *d_out, cudaStream_t s) {
         count_launches(1);
         for (const auto &sp : b->splits) {  // partial sums of this launch's split captures
             if (sp.fact != f) continue;
-            const unsigned blocks = (unsigned)std::min<uint64_t>((sp.nvox + 255) / 256, 152ull * 8);
-            reduce_splits_kernel<false, false><<<blocks, 256, 0, ls>>>(
-                b->d_scratch + sp.part_off, d_out + sp.out_off, sp.nvox, sp.splits, sp.scale);
-            count_launches(1);
+            launch_reduce_splits(b->d_scratch + sp.part_off, d_out + sp.out_off, sp.nvox, sp.splits,
+                                 sp.scale, false, ls);
         }
         BPGB_CUDA_TRY(cudaGetLastError());
     }
@@ -2992,10 +3074,7 @@ extern "C" int bpgb_backproject_noalloc(const float *d_H, uint32_t T, uint32_t h
     BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3((unsigned)(ntiles * splits)), dim3(threads), args, smem, s));
     count_launches(1);
     if (a.splits > 1) {
-        const unsigned blocks = (unsigned)std::min<uint64_t>((a.nvox + 255) / 256, 152ull * 8);
-        reduce_splits_kernel<false, false><<<blocks, 256, 0, s>>>(partial, d_volume, a.nvox,
-                                                                 a.splits, 1.0f);
-        count_launches(1);
+        launch_reduce_splits(partial, d_volume, a.nvox, a.splits, 1.0f, false, s);
         BPGB_CUDA_TRY(cudaGetLastError());
     }
     BPGB_CUDA_TRY(cudaMemcpyAsync(h, diag, sizeof(h), cudaMemcpyDeviceToHost, s));

@@ -14,6 +14,14 @@ namespace bpgb {
 constexpr float kMagic = 12582912.0f;
 constexpr uint32_t kMagicBits = 0x4B400000u;
 
+// The factor of a capture's stored rows: `scale`, or *d_absmax / target when d_absmax is set
+// (read on the device).
+__device__ __forceinline__ float scale_of(float scale, const float *d_absmax, float target) {
+    if (!d_absmax) return scale;
+    const float m = *d_absmax;
+    return m > 0.0f ? m / target : 1.0f;
+}
+
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }

@@ -124,7 +124,8 @@ int fast_plan_execute(FastPlan *fp, const void *d_H, void *d_out, cudaStream_t s
 int fast_plan_dump_bins(FastPlan *fp, const int64_t *d_ids, int64_t n, int32_t *d_bins,
                         cudaStream_t stream);
 int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const uint32_t *d_list,
-                            const uint32_t *d_count, uint32_t max_tiles, cudaStream_t stream);
+                            const uint32_t *d_count, uint32_t max_tiles, cudaStream_t stream,
+                            const float *d_absmax = nullptr, float target = 0.0f);
 int fast_plan_select_tiles(FastPlan *fp, const float *d_score, const uint32_t *block_dims,
                            uint32_t block_size, float threshold, uint32_t *d_list,
                            uint32_t *d_count, cudaStream_t stream);
@@ -136,6 +137,17 @@ int fast_plan_tables(const FastPlan *fp, float *host_out, uint64_t capacity, uin
 int fast_plan_check(FastPlan *fp, uint64_t *violations, uint64_t *timeouts);
 void fast_plan_free(FastPlan *fp);
 int wait_timeout_probe(uint32_t limit, int *timed_out);
+
+// bpgb_plan_execute_tiles and bpgb_upsample_trilinear with the stored rows' factor
+// (*d_absmax / target, as bpgb_volume_scale) applied to what they write; the tile list needs a
+// plan with pair splits, whose reduction applies it.
+int plan_execute_tiles_scaled(bpgb_plan plan, const void *d_H, void *d_volume,
+                              const uint32_t *d_tile_list, const uint32_t *d_tile_count,
+                              uint32_t max_tiles, const float *d_absmax, float target,
+                              cudaStream_t stream);
+int upsample_scaled(const float *d_coarse, const uint32_t *coarse_dims, float *d_fine,
+                    const uint32_t *fine_dims, const float *d_absmax, float target,
+                    cudaStream_t stream);
 
 // ---- phasor (phasor.cu) -------------------------------------------------------
 int launch_phasor_pulse(const float *d_H, uint64_t rows, uint32_t T, uint32_t in_pitch,

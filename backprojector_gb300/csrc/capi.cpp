@@ -267,6 +267,20 @@ struct bpgb_plan_s {
     cudaStream_t last_stream = nullptr;
 };
 
+int bpgb::plan_execute_tiles_scaled(bpgb_plan plan, const void *d_H, void *d_volume,
+                                    const uint32_t *d_tile_list, const uint32_t *d_tile_count,
+                                    uint32_t max_tiles, const float *d_absmax, float target,
+                                    cudaStream_t stream) {
+    clear_error();
+    if (!plan) return set_error(BPGB_ERR_INVALID_ARGUMENT, "plan is null");
+    if (!d_volume || !d_H) return set_error(BPGB_ERR_INVALID_ARGUMENT, "null buffer");
+    if (plan->algo != BPGB_ALGO_FAST || !plan->fast)
+        return set_error(BPGB_ERR_UNSUPPORTED, "tile-list launches need a FAST plan");
+    plan->last_stream = stream;
+    return fast_plan_execute_tiles(plan->fast, d_H, d_volume, d_tile_list, d_tile_count, max_tiles,
+                                   stream, d_absmax, target);
+}
+
 extern "C" {
 
 int bpgb_abi_version(void) { return BPGB_ABI_VERSION; }
@@ -415,15 +429,8 @@ int bpgb_plan_execute(bpgb_plan plan, const void *d_H, void *d_volume, void *str
 int bpgb_plan_execute_tiles(bpgb_plan plan, const void *d_H, void *d_volume,
                             const uint32_t *d_tile_list, const uint32_t *d_tile_count,
                             uint32_t max_tiles, void *stream) {
-    clear_error();
-    if (!plan) return set_error(BPGB_ERR_INVALID_ARGUMENT, "plan is null");
-    if (!d_volume || !d_H) return set_error(BPGB_ERR_INVALID_ARGUMENT, "null buffer");
-    if (plan->algo != BPGB_ALGO_FAST || !plan->fast)
-        return set_error(BPGB_ERR_UNSUPPORTED, "tile-list launches need a FAST plan");
-    cudaStream_t s = (cudaStream_t)stream;
-    plan->last_stream = s;
-    return fast_plan_execute_tiles(plan->fast, d_H, d_volume, d_tile_list, d_tile_count,
-                                   max_tiles, s);
+    return plan_execute_tiles_scaled(plan, d_H, d_volume, d_tile_list, d_tile_count, max_tiles,
+                                     nullptr, 0.0f, (cudaStream_t)stream);
 }
 
 int bpgb_plan_select_tiles(bpgb_plan plan, const float *d_block_score,

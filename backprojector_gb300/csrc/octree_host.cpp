@@ -31,6 +31,7 @@ struct Layer {
 struct bpgb_octree_s {
     uint32_t fine[3] = {0, 0, 0}, coarse[3] = {0, 0, 0}, tile[3] = {0, 0, 0};
     uint32_t tiles = 0, in_channels = 2, pair_splits = 8;
+    bool split = true;  // the fine plan splits its pairs
     uint64_t P = 0;
     uint32_t T = 0, pitch16 = 0;
     int h_dtype = BPGB_DTYPE_F16;
@@ -158,6 +159,7 @@ int bpgb_octree_create(bpgb_octree *out, const bpgb_pair *pairs, uint64_t num_pa
     bpgb_plan_info info;
     bpgb_plan_get_info(oc->sparse_plan, &info);
     oc->tiles = 1;
+    oc->split = info.pair_splits > 1;
     for (int k = 0; k < 3; k++) {
         oc->tile[k] = info.tile[k];
         if (info.tile[k] % kBlock)
@@ -290,15 +292,20 @@ int bpgb_octree_reconstruct(bpgb_octree oc, const float *d_H, float *d_volume, v
         in = oc->Y[li];
         xs = 16;
     }
-    if ((st = bpgb_upsample_trilinear(oc->coarse_vol, oc->coarse, d_volume, oc->fine, s))) return st;
+    // FP16 rows: the fill and the fine pass's reduction of its pair splits write the volume in
+    // the capture's units; without splits a last pass scales it
+    const bool fused = f16 && oc->split;
+    const float *absmax = fused ? oc->absmax : nullptr;
+    if ((st = upsample_scaled(oc->coarse_vol, oc->coarse, d_volume, oc->fine, absmax, kHTarget, s)))
+        return st;
     const uint32_t blocks[3] = {oc->coarse[0], oc->coarse[1], oc->coarse[2]};
     if ((st = bpgb_plan_select_tiles(oc->sparse_plan, oc->logits, blocks, kBlock, oc->logit_lo,
                                      oc->tile_list, oc->tile_count, s)))
         return st;
-    if ((st = bpgb_plan_execute_tiles(oc->sparse_plan, rows, d_volume, oc->tile_list,
-                                      oc->tile_count, oc->tiles, s)))
+    if ((st = plan_execute_tiles_scaled(oc->sparse_plan, rows, d_volume, oc->tile_list,
+                                        oc->tile_count, oc->tiles, absmax, kHTarget, s)))
         return st;
-    if (f16) {
+    if (f16 && !fused) {
         const uint64_t n = (uint64_t)oc->fine[0] * oc->fine[1] * oc->fine[2];
         if ((st = bpgb_volume_scale(d_volume, n, 1.0f, oc->absmax, kHTarget, s))) return st;
     }
