@@ -1251,44 +1251,37 @@ __global__ void __launch_bounds__(288, kFactCtas)
 }
 
 // ---- partial sums of pair splits -------------------------------------------------------
-// A voxel's sum over its splits: sums of kSegment consecutive splits, each in split order,
-// added in order (Kahan-compensated sums: one chain over all splits).  Both reductions below
-// form it the same way, so a tile-list voxel equals the full-volume one bit for bit.
-constexpr uint32_t kSegment = 8;
+// A voxel's sum over its splits is formed in split order (optionally Kahan-compensated), in
+// both reductions below, so a tile-list voxel equals the full-volume one bit for bit.
+constexpr uint32_t kSegment = 8;  // splits loaded together
 
-// Splits [k0, min(k0 + kSegment, splits)) of 4 floats; load(k) is split k's value.
-template <typename Load>
-__device__ __forceinline__ float4 segment_sum(uint32_t k0, uint32_t splits, Load &&load) {
-    float4 v[kSegment];  // all loads in flight before the first add
-#pragma unroll
-    for (uint32_t k = 0; k < kSegment; k++)
-        v[k] = k0 + k < splits ? load(k0 + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 s = v[0];
-#pragma unroll
-    for (uint32_t k = 1; k < kSegment; k++)
-        if (k0 + k < splits) s.x += v[k].x, s.y += v[k].y, s.z += v[k].z, s.w += v[k].w;
-    return s;
+__device__ __forceinline__ void add4(float4 &s, float4 v) {
+    s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
 }
 
+// 4 floats; load(k) is split k's value
 template <bool KAHAN, typename Load>
 __device__ __forceinline__ float4 splits_sum(uint32_t splits, Load &&load) {
-    if (KAHAN) {
-        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = s;
-        for (uint32_t k = 0; k < splits; k++) {
-            const float4 x = load(k);
-            kahan_add(s.x, c.x, x.x);
-            kahan_add(s.y, c.y, x.y);
-            kahan_add(s.z, c.z, x.z);
-            kahan_add(s.w, c.w, x.w);
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = s;
+    for (uint32_t k0 = 0; k0 < splits; k0 += kSegment) {
+        float4 v[kSegment];  // all loads in flight before the first add
+#pragma unroll
+        for (uint32_t k = 0; k < kSegment; k++)
+            if (k0 + k < splits) v[k] = load(k0 + k);
+#pragma unroll
+        for (uint32_t k = 0; k < kSegment; k++) {
+            if (k0 + k >= splits) break;
+            if (KAHAN) {
+                kahan_add(s.x, c.x, v[k].x);
+                kahan_add(s.y, c.y, v[k].y);
+                kahan_add(s.z, c.z, v[k].z);
+                kahan_add(s.w, c.w, v[k].w);
+            } else {
+                add4(s, v[k]);
+            }
         }
-        return make_float4(s.x - c.x, s.y - c.y, s.z - c.z, s.w - c.w);
     }
-    float4 s = segment_sum(0, splits, load);
-    for (uint32_t k = kSegment; k < splits; k += kSegment) {
-        const float4 t = segment_sum(k, splits, load);
-        s.x += t.x, s.y += t.y, s.z += t.z, s.w += t.w;
-    }
-    return s;
+    return KAHAN ? make_float4(s.x - c.x, s.y - c.y, s.z - c.z, s.w - c.w) : s;
 }
 
 // n floats at p + i, fewer than 4 at the end; `vec`: p is 16-byte aligned
@@ -1314,13 +1307,13 @@ __device__ __forceinline__ float4 scaled(float4 v, float f) {
     return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
 }
 
-// out[i] = scale * (sum of partial[s][i] over the splits), i < n floats.  A block takes
-// 256 groups of 4 floats, one per thread; with more than kSegment splits and too few groups
-// for a GPU full of threads (`rows`), kReduceX groups, whose segments are summed by the other
-// rows of threads and added by row 0 in order.  Latency bounds it (each float is read once):
-// 4,096 voxels x 64 splits 8.7 -> 3.6 us, 262,144 voxels x 7 splits 4.6 -> 3.9 us against one
-// thread and one chain of loads per voxel.
-constexpr uint32_t kReduceX = 32, kReduceY = 8;
+// out[i] = scale * (sum of partial[s][i] over the splits), i < n floats.  A block takes 256
+// groups of 4 floats, one per thread; with more than kSegment splits and too few groups for a
+// GPU full of threads (`rows`), kReduceX groups, whose splits its kReduceY rows of threads
+// load together and row 0 adds in order.  Latency bounds it (each float is read once):
+// against one thread and one chain of loads per voxel, 262,144 voxels x 7 splits took 4.6 ->
+// 3.9 us, and a whole pass over 4,096 voxels x 64 splits 14.3 -> 12.3 us (32 x 8 threads: 14.3).
+constexpr uint32_t kReduceX = 16, kReduceY = 16, kReduceK = 4;  // kReduceK splits per thread
 template <bool KAHAN>
 __global__ void __launch_bounds__(kReduceX *kReduceY)
     reduce_splits_kernel(const float *__restrict__ partial, float *__restrict__ out, uint64_t n,
@@ -1335,25 +1328,27 @@ __global__ void __launch_bounds__(kReduceX *kReduceY)
         store4(out, i, n, vec, scaled(splits_sum<KAHAN>(splits, load), scale));
         return;
     }
-    __shared__ float4 seg[kReduceY][kReduceX];
+    __shared__ float4 part[kReduceY * kReduceK][kReduceX];
     const uint64_t q = (uint64_t)blockIdx.x * kReduceX + threadIdx.x, i = 4 * q;
     float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (uint32_t k0 = 0; k0 < splits; k0 += kReduceY * kSegment) {
-        const uint32_t k = k0 + threadIdx.y * kSegment;
-        if (q < quads && k < splits)
-            seg[threadIdx.y][threadIdx.x] = segment_sum(
-                k, splits, [&](uint32_t s) { return load4(partial + s * n, i, n, vp); });
-        __syncthreads();
-        if (threadIdx.y == 0) {
-            for (uint32_t y = 0; y < kReduceY && k0 + y * kSegment < splits; y++) {
-                const float4 t = seg[y][threadIdx.x];
-                if (k0 + y == 0)
-                    sum = t;
-                else
-                    sum.x += t.x, sum.y += t.y, sum.z += t.z, sum.w += t.w;
-            }
+    for (uint32_t k0 = 0; k0 < splits; k0 += kReduceY * kReduceK) {
+        const uint32_t nk = min(splits - k0, kReduceY * kReduceK);
+        if (k0 > 0) __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < kReduceK; j++) {
+            const uint32_t k = threadIdx.y + j * kReduceY;
+            if (q < quads && k < nk) part[k][threadIdx.x] = load4(partial + (k0 + k) * n, i, n, vp);
         }
         __syncthreads();
+        if (threadIdx.y == 0)
+            for (uint32_t k = 0; k < nk; k += 8) {
+                float4 v[8];
+#pragma unroll
+                for (uint32_t j = 0; j < 8; j++) v[j] = part[k + j][threadIdx.x];
+#pragma unroll
+                for (uint32_t j = 0; j < 8; j++)
+                    if (k + j < nk) add4(sum, v[j]);
+            }
     }
     if (threadIdx.y == 0 && q < quads) store4(out, i, n, vec, scaled(sum, scale));
 }
@@ -2023,7 +2018,9 @@ int fast_plan_build(FastPlan **out, const bpgb_pair *d_pairs, uint64_t P,
     const uint64_t ngroups = (ntiles + a.groups - 1) / a.groups;  // CTAs per pair split
     const uint64_t items = fast_items(a);
     uint64_t splits = opt.pair_splits > 0 ? (uint64_t)opt.pair_splits
-                                          : auto_splits(ngroups, items, (uint32_t)sm_count, occ);
+                      : opt.pair_splits < 0  // fill two rounds: does not move with the rule
+                          ? std::max<uint64_t>(1, (2ull * sm_count * occ + ngroups - 1) / ngroups)
+                          : auto_splits(ngroups, items, (uint32_t)sm_count, occ);
     splits = std::max<uint64_t>(1, std::min<uint64_t>(splits, items));
     if (ngroups * splits >= (1ull << 31)) {
         fast_plan_free(fp);

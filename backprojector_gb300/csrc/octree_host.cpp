@@ -141,7 +141,8 @@ int bpgb_octree_create(bpgb_octree *out, const bpgb_pair *pairs, uint64_t num_pa
     po.h_scale = 1.0f;
     po.checked = 0;
     po.tile = -1;
-    po.pair_splits = 0;
+    // the network's decisions move with the last bit of the coarse sums: a fixed division
+    po.pair_splits = -1;
     po.chunk = 0;
     po.stages = 0;
     int st = bpgb_plan_create(&oc->coarse_plan, pairs, num_pairs, T, oc->coarse, volume_zero_pos,

@@ -381,8 +381,11 @@ class Reconstructor:
             self.rows = self.H
         self.coarse = torch.empty(geo.coarse, dtype=torch.float32, device=device)
         self.fine = torch.empty(geo.fine, dtype=torch.float32, device=device)
+        # pair_splits=-1: the network's decisions move with the last bit of the coarse sums, so
+        # their division over CTAs is a fixed one
         self.coarse_plan = capi.Plan(geo.pairs, geo.T, geo.coarse, geo.zero, geo.inc_coarse,
-                                     geo.t0, geo.deltaT, algo=capi.ALGO_FAST, h_dtype=h_dtype)
+                                     geo.t0, geo.deltaT, algo=capi.ALGO_FAST, h_dtype=h_dtype,
+                                     pair_splits=-1)
         # The fine plan serves both the dense reference (execute) and the block-sparse
         # pass (execute_tiles): FAST arithmetic is tile-relative, so one plan gives
         # bit-identical voxels in both.
@@ -416,7 +419,7 @@ class Reconstructor:
         inc_fill = (np.asarray(geo.inc_fine, np.float64).reshape(3, 3) * (n - 1) / (fill - 1))
         self.fill_plan = capi.Plan(geo.pairs, geo.T, self.fill_dims, geo.zero,
                                    inc_fill.astype(np.float32).reshape(-1), geo.t0, geo.deltaT,
-                                   algo=capi.ALGO_FAST, h_dtype=h_dtype)
+                                   algo=capi.ALGO_FAST, h_dtype=h_dtype, pair_splits=-1)
         self.fill_vol = torch.empty(self.fill_dims, dtype=torch.float32, device=device)
         self.score = torch.empty(self.blocks, dtype=torch.float32, device=device)
         self.X0 = torch.empty(int(np.prod(geo.coarse)) * 2, dtype=torch.bfloat16, device=device)
@@ -670,7 +673,8 @@ class PhasorOctree:
         ic = (np.asarray(inc, np.float64).reshape(3, 3) * ((n - 1) / (n // BLOCK - 1))[:, None])
         ic = ic.astype(np.float32).reshape(-1)
         common = dict(algo=capi.ALGO_FAST, h_dtype=capi.DTYPE_C64, h_pitch=h_pitch)
-        self.coarse_plan = capi.Plan(pairs, T, self.coarse, zero, ic, t0, deltaT, **common)
+        self.coarse_plan = capi.Plan(pairs, T, self.coarse, zero, ic, t0, deltaT, pair_splits=-1,
+                                     **common)
         self.fine_plan = capi.Plan(pairs, T, self.fine, zero, inc, t0, deltaT, tile=fine_tile,
                                    pair_splits=fine_splits, **common)
         info = self.fine_plan.info()

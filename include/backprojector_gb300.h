@@ -89,7 +89,9 @@ typedef struct bpgb_options {
     int32_t tile;        /* tile preset index (-1 = tuned default); 10-12: small tiles for
                             block-sparse passes, 13: four 8^3 tiles per CTA (real rows,
                             plain sums) */
-    int32_t pair_splits; /* CTAs sharing one voxel tile over disjoint pair ranges (0 = auto) */
+    int32_t pair_splits; /* CTAs sharing one voxel tile over disjoint pair ranges (0 = auto,
+                            negative = plans: as many as fill two rounds of CTAs, so that sums
+                            do not move with the automatic choice) */
     int32_t checked;     /* 1 = clamp and count out-of-window bins (tests) */
     uint32_t spin_limit; /* bounded mbarrier waits: polls before giving up (0 = default) */
     int32_t chunk;       /* FAST: SPAD rows per pipeline stage, 1..64 (0 = from the preset;
