@@ -26,9 +26,10 @@
 //     tile centre (bin units) and the accumulators, all as voxel pairs.  Per row and
 //     voxel pair (sm_100 packed FP32x2 ops, one instruction for two voxels):
 //       dz = vk - ck; q = dz*dz + D; r = rsqrt(q) (MUFU, per voxel);
-//       x = q*r + A; y = x + row constant; z = y + 1.5*2^23 (round to nearest);
-//     then one shifted-add per voxel forms the shared address and one load gathers.
-//     That is 6 FP32x2 + 2 MUFU + 2 address + 2 gathers = 12 issue slots per two updates;
+//       y = q*r + (A + row constant); n = y * 2^-149 (subnormal: rounds to the nearest bin);
+//       a = n * element size + row address: the bits are the shared address;
+//     then one load per voxel gathers.  That is 6 FP32x2 + accumulate + 2 MUFU + 2 gathers = 11
+//     issue slots per two updates;
 //     FP16/BF16 rows accumulate with sm_100's one-op mixed-precision add.
 //   * Stages are handed over with mbarriers (full: TMA bytes + producer arrive; empty:
 //     one arrive per consumer warp; the producer sleeps briefly between its polls, so
@@ -261,30 +262,46 @@ __device__ __forceinline__ uint32_t window_bits(float vk, float D, float A, floa
 // loads written as C++ dereferences of the generic base pointer ran 9-12% slower (dense
 // 256^3 79.3 against 71.9 ms, the 64-capture batch 115.5 against 101.3 ms).
 template <typename T>
-__device__ __forceinline__ T lds(const unsigned char *smem, uint32_t off);
+__device__ __forceinline__ T lds(uint32_t off);
 template <>
-__device__ __forceinline__ float lds<float>(const unsigned char *smem, uint32_t off) {
+__device__ __forceinline__ float lds<float>(uint32_t off) {
     float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_addr(smem) + off));
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(off));
     return v;
 }
 template <>
-__device__ __forceinline__ unsigned short lds<unsigned short>(const unsigned char *smem, uint32_t off) {
+__device__ __forceinline__ unsigned short lds<unsigned short>(uint32_t off) {
     unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(smem_addr(smem) + off));
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(off));
     return v;
 }
 template <>
-__device__ __forceinline__ uint32_t lds<uint32_t>(const unsigned char *smem, uint32_t off) {
+__device__ __forceinline__ uint32_t lds<uint32_t>(uint32_t off) {
     uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr(smem) + off));
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(off));
     return v;
 }
 template <>
-__device__ __forceinline__ float2 lds<float2>(const unsigned char *smem, uint32_t off) {
+__device__ __forceinline__ float2 lds<float2>(uint32_t off) {
     float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_addr(smem) + off));
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(off));
     return v;
+}
+
+// Shared addresses of the bins nearest to the two window positions y >= 0: the product with the
+// smallest subnormal, 2^-149, rounds y to the nearest integer (to even on ties) of that
+// spacing, so its bits are the bin; one FMA on those subnormals scales it by the element size
+// and adds the row's base address, itself a float of those bits.  Two packed instructions for
+// two addresses, where adding 1.5 x 2^23 and a shift-and-add for each take three: 256^3 voxels
+// 68.8 -> 67.4 ms, 64^3 318 -> 309 us, learned octree 3.48 -> 3.41 ms, the same bins.
+__device__ __forceinline__ uint2 bin_addresses(float2 y, uint32_t esz, float2 base) {
+    const float unit = __uint_as_float(1u);
+    const float2 n = __fmul2_rn(y, make_float2(unit, unit));
+    const float2 t = __ffma2_rn(n, make_float2((float)esz, (float)esz), base);
+    return make_uint2(__float_as_uint(t.x), __float_as_uint(t.y));
+}
+__device__ __forceinline__ float2 address_pair(uint32_t a) {
+    return make_float2(__uint_as_float(a), __uint_as_float(a));
 }
 
 __device__ __forceinline__ void kahan_add(float &sum, float &comp, float x) {
@@ -304,8 +321,8 @@ struct Pair<float> {
     static constexpr bool kCplx = false;
     float2 a;
     __device__ __forceinline__ void zero() { a = make_float2(0.0f, 0.0f); }
-    __device__ __forceinline__ void gather2(const unsigned char *sm, uint32_t p0, uint32_t p1) {
-        const float v0 = lds<float>(sm, p0), v1 = lds<float>(sm, p1);
+    __device__ __forceinline__ void gather2(uint32_t p0, uint32_t p1) {
+        const float v0 = lds<float>(p0), v1 = lds<float>(p1);
         a = __fadd2_rn(a, make_float2(v0, v1));
     }
     __device__ __forceinline__ void fold(Pair &comp, const Pair &part) {
@@ -327,8 +344,8 @@ struct PairHalf {
     static constexpr bool kCplx = false;
     float2 a;
     __device__ __forceinline__ void zero() { a = make_float2(0.0f, 0.0f); }
-    __device__ __forceinline__ void gather2(const unsigned char *sm, uint32_t p0, uint32_t p1) {
-        const unsigned short h0 = lds<unsigned short>(sm, p0), h1 = lds<unsigned short>(sm, p1);
+    __device__ __forceinline__ void gather2(uint32_t p0, uint32_t p1) {
+        const unsigned short h0 = lds<unsigned short>(p0), h1 = lds<unsigned short>(p1);
         if (IS_BF16) {
             asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(a.x) : "h"(h0));
             asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(a.y) : "h"(h1));
@@ -360,8 +377,8 @@ struct Pair<float2> {
     static constexpr bool kCplx = true;
     float2 a0, a1;
     __device__ __forceinline__ void zero() { a0 = a1 = make_float2(0.0f, 0.0f); }
-    __device__ __forceinline__ void gather2(const unsigned char *sm, uint32_t p0, uint32_t p1) {
-        const float2 v0 = lds<float2>(sm, p0), v1 = lds<float2>(sm, p1);
+    __device__ __forceinline__ void gather2(uint32_t p0, uint32_t p1) {
+        const float2 v0 = lds<float2>(p0), v1 = lds<float2>(p1);
         a0 = __fadd2_rn(a0, v0);
         a1 = __fadd2_rn(a1, v1);
     }
@@ -399,9 +416,9 @@ struct Pair<__half2> {
             : "+f"(acc.x), "+f"(acc.y)
             : "r"(w));
     }
-    __device__ __forceinline__ void gather2(const unsigned char *sm, uint32_t p0, uint32_t p1) {
-        add_c16(a0, lds<uint32_t>(sm, p0));
-        add_c16(a1, lds<uint32_t>(sm, p1));
+    __device__ __forceinline__ void gather2(uint32_t p0, uint32_t p1) {
+        add_c16(a0, lds<uint32_t>(p0));
+        add_c16(a1, lds<uint32_t>(p1));
     }
     __device__ __forceinline__ void fold(Pair &comp, const Pair &part) {
         kahan_add(a0.x, comp.a0.x, part.a0.x);
@@ -525,9 +542,7 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
     constexpr int NP = K / 2;
     // stage entries per producer lane
     constexpr uint32_t kLane = GROUPED ? kMaxGroupEntries / 32 : kMaxChunk / 32;
-    unsigned char *const smem_raw = sh.smem_raw;
     unsigned char *const stage_base = sh.stage_base;
-    const uint32_t pad = sh.pad;
     uint64_t *const full_bar = sh.full_bar;
     uint64_t *const empty_bar = sh.empty_bar;
     int &abort_flag = *sh.abort_flag;
@@ -691,7 +706,7 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
     uint32_t cw = warp - 1, grp = 0;
     bool live = true;
     unsigned char *tab_base = stage_base;
-    uint32_t data_base = pad;  // offset from smem_raw
+    uint32_t data_base = smem_addr(stage_base);
     if constexpr (GROUPED) {
         const uint32_t twarps = a.warp[0] * a.warp[1] * a.warp[2];
         grp = cw / twarps;
@@ -811,7 +826,8 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
                 const float4 r1 = table[2 * j + 1];  // (-c_k, -c_k, ew, ew)
                 nk = make_float2(r1.x, r1.y);
             }
-            const uint32_t rbase = data + j * a.row_bytes - kMagicBits * esz;
+            const uint32_t rbase = data + j * a.row_bytes;
+            const float2 base2 = address_pair(rbase);
 #pragma unroll
             for (int p = 0; p < NP; p++) {
                 // laser leg + row constant ahead of the rsqrt: one dependent op after it
@@ -825,25 +841,20 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
                 }
                 const float2 r = make_float2(rsqrt_approx(q.x), rsqrt_approx(q.y));
                 const float2 y = __ffma2_rn(q, r, Ae);
-                const float2 z = __fadd2_rn(y, magic2);
-                uint32_t b0 = __float_as_uint(z.x), b1 = __float_as_uint(z.y);
+                uint2 at;
                 if (CHECKED) {
-                    const uint32_t r0i = b0 - kMagicBits, r1i = b1 - kMagicBits;
-                    if (r0i >= a.W) {
-                        violations++;
-                        b0 = kMagicBits + ((int32_t)r0i < 0 ? 0u : a.W - 1);
-                    }
-                    if (r1i >= a.W) {
-                        violations++;
-                        b1 = kMagicBits + ((int32_t)r1i < 0 ? 0u : a.W - 1);
-                    }
+                    const float2 z = __fadd2_rn(y, magic2);
+                    uint32_t b0 = __float_as_uint(z.x) - kMagicBits, b1 = __float_as_uint(z.y) - kMagicBits;
+                    if (b0 >= a.W) violations++, b0 = (int32_t)b0 < 0 ? 0u : a.W - 1;
+                    if (b1 >= a.W) violations++, b1 = (int32_t)b1 < 0 ? 0u : a.W - 1;
+                    at = make_uint2(rbase + (b0 << PairT::kShift), rbase + (b1 << PairT::kShift));
+                } else {
+                    at = bin_addresses(y, esz, base2);
                 }
-                const uint32_t p0 = rbase + (b0 << PairT::kShift);
-                const uint32_t p1 = rbase + (b1 << PairT::kShift);
                 if (KAHAN)
-                    part[p].gather2(smem_raw, p0, p1);
+                    part[p].gather2(at.x, at.y);
                 else
-                    acc[p].gather2(smem_raw, p0, p1);
+                    acc[p].gather2(at.x, at.y);
             }
         }
         __syncwarp();
@@ -909,9 +920,7 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
     using PairT = Pair<HT>;
     constexpr uint32_t esz = PairT::kEsz;
     constexpr int K = 8, NP = K / 2;
-    unsigned char *const smem_raw = sh.smem_raw;
     unsigned char *const stage_base = sh.stage_base;
-    const uint32_t pad = sh.pad;
     uint64_t *const full_bar = sh.full_bar;
     uint64_t *const empty_bar = sh.empty_bar;
     int &abort_flag = *sh.abort_flag;
@@ -1076,7 +1085,7 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
         const uint32_t ncl = (uint32_t)(a.L - l0 < (uint64_t)cl ? a.L - l0 : (uint64_t)cl);
         const float4 *table =
             reinterpret_cast<const float4 *>(stage_base + (size_t)stage * a.stage_bytes);
-        const uint32_t data = pad + stage * a.stage_bytes + a.table_bytes;  // offset from smem_raw
+        const uint32_t data = smem_addr(stage_base) + stage * a.stage_bytes + a.table_bytes;
         if (sb != cur_sb) {
 #pragma unroll
             for (uint32_t si = 0; si < kFactS; si++) legs(table[cl + si], B[si]);
@@ -1087,24 +1096,21 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
             legs(table[lj], A);
 #pragma unroll
             for (uint32_t si = 0; si < kFactS; si++) {
-                const uint32_t rbase = data + (lj * kFactS + si) * a.row_bytes - kMagicBits * esz;
+                const uint32_t rbase = data + (lj * kFactS + si) * a.row_bytes;
+                const float2 base2 = address_pair(rbase);
 #pragma unroll
                 for (int p = 0; p < NP; p++) {
-                    const float2 z = __fadd2_rn(__fadd2_rn(A[p], B[si][p]), magic2);
-                    uint32_t b0 = __float_as_uint(z.x), b1 = __float_as_uint(z.y);
+                    const float2 y = __fadd2_rn(A[p], B[si][p]);
                     if (CHECKED) {
-                        const uint32_t r0i = b0 - kMagicBits, r1i = b1 - kMagicBits;
-                        if (r0i >= a.W) {
-                            violations++;
-                            b0 = kMagicBits + ((int32_t)r0i < 0 ? 0u : a.W - 1);
-                        }
-                        if (r1i >= a.W) {
-                            violations++;
-                            b1 = kMagicBits + ((int32_t)r1i < 0 ? 0u : a.W - 1);
-                        }
+                        const float2 z = __fadd2_rn(y, magic2);
+                        uint32_t b0 = __float_as_uint(z.x) - kMagicBits, b1 = __float_as_uint(z.y) - kMagicBits;
+                        if (b0 >= a.W) violations++, b0 = (int32_t)b0 < 0 ? 0u : a.W - 1;
+                        if (b1 >= a.W) violations++, b1 = (int32_t)b1 < 0 ? 0u : a.W - 1;
+                        acc[p].gather2(rbase + (b0 << PairT::kShift), rbase + (b1 << PairT::kShift));
+                    } else {
+                        const uint2 at = bin_addresses(y, esz, base2);
+                        acc[p].gather2(at.x, at.y);
                     }
-                    acc[p].gather2(smem_raw, rbase + (b0 << PairT::kShift),
-                                   rbase + (b1 << PairT::kShift));
                 }
             }
         }
