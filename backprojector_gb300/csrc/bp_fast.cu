@@ -1732,7 +1732,7 @@ void *select_fact_kernel(int dtype, bool checked) {
 int fast_args(FastArgs &a, const FastConfig &cfg, const Volume &vol, const double hd[3],
               bool confocal, double dT, double t0, uint64_t L, uint64_t S, uint32_t T,
               uint32_t esz, bool kahan, uint32_t chunk_req, uint32_t stages_req,
-              std::string *why, uint32_t bw_fixed = 0, bool fact = false) {
+              std::string *why, bool fact = false) {
     auto no = [&](const std::string &m) {
         if (why) *why = m;
         return BPGB_ERR_UNSUPPORTED;
@@ -1783,13 +1783,8 @@ int fast_args(FastArgs &a, const FastConfig &cfg, const Volume &vol, const doubl
     // aligned down, so the window carries one more alignment of slack
     const uint32_t w_need = (uint32_t)std::ceil(span) + (fact ? 2 : 1) * a.align;
     const uint32_t bw_align = 128 / esz;
-    if (bw_fixed) {  // one TMA box width shared by several captures (batches)
-        a.BW = bw_fixed;
-        a.nbox = (w_need + bw_fixed - 1) / bw_fixed;
-    } else {
-        a.nbox = (w_need + 255) / 256;
-        a.BW = ((w_need + a.nbox - 1) / a.nbox + bw_align - 1) / bw_align * bw_align;
-    }
+    a.nbox = (w_need + 255) / 256;
+    a.BW = ((w_need + a.nbox - 1) / a.nbox + bw_align - 1) / bw_align * bw_align;
     if (a.BW > 256) return no("window box too wide");
     a.W = a.BW * a.nbox;
     a.row_bytes = a.W * esz;
@@ -1950,7 +1945,7 @@ int fast_plan_build(FastPlan **out, const bpgb_pair *d_pairs, uint64_t P,
     std::string why;
     int st = fast_args(a, cfg, vol, hd, confocal, bp.dT, bp.t0, L, fz.S, bp.T, esz,
                        opt.accum == BPGB_ACCUM_KAHAN, opt.chunk > 0 ? (uint32_t)opt.chunk : 0,
-                       opt.stages > 0 ? (uint32_t)opt.stages : 0, &why, 0, fact);
+                       opt.stages > 0 ? (uint32_t)opt.stages : 0, &why, fact);
     if (st) return no(why);
     a.out_scale = opt.h_scale != 0.0f ? opt.h_scale : 1.0f;
     if (opt.spin_limit) a.spin_limit = opt.spin_limit;
@@ -2349,13 +2344,20 @@ struct BatchUnit {
     uint32_t cap, tile, split;
 };
 
+// The packed rows' tensor maps, one per box width of 128, 256 .. 1024 bytes (at most 256
+// elements): a capture's windows arrive in as few TMA boxes as a plan's would.
+constexpr uint32_t kBatchMaps = 8;
+struct BatchMaps {
+    CUtensorMap m[kBatchMaps];
+};
+
 // FACT: the launch over the batch's lasers x SPADs captures (factored legs); otherwise the
 // launch over the rest (per-pair legs).  Each is one persistent launch over its own
 // cost-sorted unit list with its own counters; a batch with both kinds runs the two
 // launches back to back.
 template <typename HT, bool CHECKED, bool PLANAR, bool FACT>
 __global__ void __launch_bounds__(288, FACT ? kFactCtas : 3)
-    bp_batch_kernel(const __grid_constant__ CUtensorMap tmap, const BatchCap *__restrict__ caps,
+    bp_batch_kernel(const __grid_constant__ BatchMaps maps, const BatchCap *__restrict__ caps,
                     const BatchUnit *__restrict__ units, uint32_t n_units,
                     const float4 *__restrict__ tables, float *__restrict__ out,
                     float *__restrict__ scratch, unsigned long long *__restrict__ diag,
@@ -2390,14 +2392,15 @@ __global__ void __launch_bounds__(288, FACT ? kFactCtas : 3)
         __syncthreads();
         if (*(volatile int *)&abort_flag) break;
         const float4 *tab = tables + cap_s.tab_off;
+        const CUtensorMap *tmap = &maps.m[cap_s.a.BW * Pair<HT>::kEsz / 128 - 1];
         // split captures write partial sums (reduced after the launch), the rest the volume
         float *dst = cap_s.a.splits > 1 ? scratch + cap_s.part_off : out + cap_s.out_off;
         if constexpr (FACT)
-            ok = fact_unit<HT, CHECKED>(cap_s.a, &tmap, tab, tab + cap_s.a.S, dst, diag, u.tile,
+            ok = fact_unit<HT, CHECKED>(cap_s.a, tmap, tab, tab + cap_s.a.S, dst, diag, u.tile,
                                         u.split, (uint32_t)cap_s.row_base, step, sh);
         else
             ok = fast_unit<HT, 8, false, CHECKED, PLANAR, kBatchRows, false>(
-                cap_s.a, &tmap, tab, tab + cap_s.a.S, dst, diag, u.tile, u.split,
+                cap_s.a, tmap, tab, tab + cap_s.a.S, dst, diag, u.tile, u.split,
                 (uint32_t)cap_s.row_base, step, sh);
         if (!ok) *(volatile int *)&abort_flag = 1;
     }
@@ -2436,6 +2439,7 @@ struct BatchPlan {
     int dtype = BPGB_DTYPE_F32;
     bool checked = false, planar = false;
     uint32_t n = 0, pitch = 0, stages = 0, chunk = 0, smem = 0, grid = 0, n_units = 0;
+    uint32_t boxes = 0;  // bit k: a capture stages boxes of (k + 1) x 128 bytes
     // units [0, n_units - n_fact) run per-pair legs, the last n_fact factored legs (a
     // second launch with grid_fact CTAs and the counters d_sched[2..3]); each launch has
     // its own stage ring (ring[0] per-pair, ring[1] factored)
@@ -2490,15 +2494,13 @@ int batch_execute(BatchPlan *b, const void *d_H, float *d_out, cudaStream_t s) {
     if (!d_H || !d_out) return set_error(BPGB_ERR_INVALID_ARGUMENT, "null batch buffer");
     if (((uintptr_t)d_H) % 16) return set_error(BPGB_ERR_INVALID_ARGUMENT, "H must be 16-byte aligned");
     const uint32_t esz = dtype_bytes(b->dtype);
-    const cuuint64_t dims[2] = {b->pitch, b->total_rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)b->pitch * esz};
-    const cuuint32_t box[2] = {128 / esz, 1};
-    const cuuint32_t estr[2] = {1, 1};
-    CUtensorMap map;
-    CUresult r = encode_fn()(&map, tma_type(b->dtype), 2, const_cast<void *>(d_H), dims, strides, box,
-                             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return set_error(BPGB_ERR_CUDA, "cuTensorMapEncodeTiled failed (batch)");
+    BatchMaps map{};
+    for (uint32_t k = 0; k < kBatchMaps; k++)
+        if (b->boxes >> k & 1) {
+            const int st = encode_rows(&map.m[k], b->dtype, d_H, b->pitch, b->total_rows, b->pitch,
+                                       (k + 1) * 128 / esz);
+            if (st) return st;
+        }
     // With both kinds of capture the two persistent launches run concurrently: the
     // factored launch (most of the work) on `s`, the per-pair launch on the batch's side
     // stream forked from and joined back into `s` (two branches of a captured graph).
@@ -2582,7 +2584,7 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
     };
     std::vector<TableJob> tjobs;
     uint64_t tab_count = 0;
-    uint32_t max_row_bytes = 0, tmax = 0;
+    uint32_t tmax = 0;
     for (uint32_t c = 0; c < n; c++) {
         const bpgb_capture_geometry &g = caps[c];
         auto fail = [&](int code, const std::string &m) {
@@ -2611,7 +2613,7 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         for (;;) {  // the per-pair form where the factored one does not fit
             st = fast_args(a, cfg, vol, hd, confocal, g.deltaT, g.t0, L, fz.S, g.T, esz, false,
                            o.chunk > 0 ? (uint32_t)o.chunk : 0,
-                           o.stages > 0 ? (uint32_t)o.stages : 0, &why, bw, fact);
+                           o.stages > 0 ? (uint32_t)o.stages : 0, &why, fact);
             if (!st || !fact) break;
             fact = false;
         }
@@ -2619,7 +2621,7 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         a.out_scale = g.h_scale != 0.0f ? g.h_scale : 1.0f;
         a.splits = 1;
         a.spin_limit = b->spin_limit;
-        max_row_bytes = std::max(max_row_bytes, a.row_bytes);
+        b->boxes |= 1u << (a.BW * esz / 128 - 1);
         tmax = std::max(tmax, g.T);
         // tables: built on the GPU after the loop (same FP64 kernel as a plan)
         hc[c].tab_off = tab_count;
@@ -2708,11 +2710,15 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         batch_free(b);
         return set_error(BPGB_ERR_UNSUPPORTED, "widest time window does not fit in shared memory");
     }
+    uint32_t stage_bytes[2] = {0, 0};
     for (int f = 0; f < 2; f++) {
+        if (!row_bytes[f]) continue;
+        stage_bytes[f] = table_bytes_of(chunk[f]) + chunk[f] * row_bytes[f];
+        if (o.chunk <= 0)
+            stage_bytes[f] = std::max<uint32_t>(stage_bytes[f], (f ? 110 : 72) * 1024 / stages[f] / 128 * 128);
         b->ring[f].chunk = chunk[f];
         b->ring[f].stages = stages[f];
-        b->ring[f].smem =
-            row_bytes[f] ? stages[f] * (table_bytes_of(chunk[f]) + chunk[f] * row_bytes[f]) + 128 : 0;
+        b->ring[f].smem = stages[f] * stage_bytes[f] + 128;
     }
     const int shown = row_bytes[0] ? 0 : 1;  // the ring bpgb_batch_info reports
     b->chunk = chunk[shown];
@@ -2723,12 +2729,16 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
     for (uint32_t c = 0; c < n; c++) {
         FastArgs &a = hc[c].a;
         const int f = a.fact ? 1 : 0;
-        a.chunk = chunk[f];
+        uint32_t ch = chunk[f];
+        if (o.chunk <= 0)
+            while (ch + 4 <= cfg.chunk && table_bytes_of(ch + 4) + (ch + 4) * a.row_bytes <= stage_bytes[f])
+                ch += 4;
+        a.chunk = ch;
         a.stages = stages[f];
-        a.table_bytes = table_bytes_of(chunk[f]);
-        a.stage_bytes = table_bytes_of(chunk[f]) + chunk[f] * row_bytes[f];
-        a.nchunks = a.fact ? (uint32_t)((a.L + chunk[f] / kFactS - 1) / (chunk[f] / kFactS))
-                           : (uint32_t)((a.S + chunk[f] - 1) / chunk[f]);
+        a.table_bytes = table_bytes_of(ch);
+        a.stage_bytes = stage_bytes[f];
+        a.nchunks = a.fact ? (uint32_t)((a.L + ch / kFactS - 1) / (ch / kFactS))
+                           : (uint32_t)((a.S + ch - 1) / ch);
         if (fast_items(a) >= (1ull << 32)) {
             batch_free(b);
             return set_error(BPGB_ERR_UNSUPPORTED, "more than 2^32 (laser, chunk) items");
