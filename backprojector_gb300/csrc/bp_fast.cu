@@ -60,9 +60,10 @@ namespace bpgb {
 namespace {
 
 constexpr int kPlanRows = 16;  // rows per unrolled consumer iteration: plans
-constexpr int kBatchRows = 4;  // and the batch kernel
+constexpr int kBatchRows = 8;  // the batch kernel
+constexpr int kGroupRows = 8;  // and plans of several tiles per CTA
 constexpr int kC32Rows = 4;    // complex rows (FP16 pairs / complex64), whose accumulators
-constexpr int kC64Rows = 1;    // already double the registers
+constexpr int kC64Rows = 2;    // already double the registers
 constexpr uint32_t kMaxChunk = 64;                         // rows per stage (two per lane)
 constexpr uint32_t kMaxGroupEntries = 128;  // grouped stages: (tile, row) entries, four per lane
 constexpr uint32_t kMaxGroups = 4;          // tiles per CTA
@@ -660,8 +661,8 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
                         float ev[3], ew;
                         const int32_t lo = row_record(a, box_g[gi], G, lt_g[gi], ev, ew);
                         const float ek = sel3(ev[0], ev[1], ev[2], a.kax);
-                        table[2 * e] = make_float4(sel3(ev[0], ev[1], ev[2], a.oax0),
-                                                   sel3(ev[0], ev[1], ev[2], a.oax1), ew, ew);
+                        table[2 * e] = make_float4(-sel3(ev[0], ev[1], ev[2], a.oax0),
+                                                   -sel3(ev[0], ev[1], ev[2], a.oax1), ew, ew);
                         table[2 * e + 1] = make_float4(-ek, -ek, ew, ew);
                         const int32_t row = (int32_t)(row_base + l * a.S + s0 + r);
                         const uint32_t dst = data + e * a.row_bytes;
@@ -681,8 +682,8 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
                         float ev[3], ew;
                         lo[q] = row_record(a, box, G, lt, ev, ew);
                         const float ek = sel3(ev[0], ev[1], ev[2], a.kax);
-                        table[2 * e] = make_float4(sel3(ev[0], ev[1], ev[2], a.oax0),
-                                                   sel3(ev[0], ev[1], ev[2], a.oax1), ew, ew);
+                        table[2 * e] = make_float4(-sel3(ev[0], ev[1], ev[2], a.oax0),
+                                                   -sel3(ev[0], ev[1], ev[2], a.oax1), ew, ew);
                         table[2 * e + 1] = make_float4(-ek, -ek, ew, ew);
                     }
                 }
@@ -820,13 +821,17 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
         }
         // ROWS rows per unrolled iteration give the scheduler ROWS x NP independent
         // voxel-pair chains to interleave (one row for complex rows, whose accumulators
-        // already double the registers).  Measured on the 256^3 capture: 2 rows 86.7 ms,
-        // 4 rows 84.5, 8 rows 80.9, 16 rows 80.4 (the batch kernel: 4 rows best).
+        // already double the registers).  Measured: 256^3 voxels 4 rows
+        // 75.4 ms, 8 rows 73.6, 16 rows 69.6; four 8^3 tiles per CTA (learned octree) 4 rows
+        // 3.47 ms, 8 rows 3.32, 16 rows 3.38; the batch kernel 4 rows 36.96, 8 rows 36.74, 16 rows
+        // 36.91; complex64 rows (128^3) 1 row 16.14, 2 rows 16.08.
         const uint32_t jn = live ? nrows : 0u;  // a tile past the list or volume idles
-#pragma unroll(PairT::kCplx ? (PairT::kEsz == 8 ? kC64Rows : kC32Rows) : ROWS)
+#pragma unroll(PairT::kCplx ? (PairT::kEsz == 8 ? kC64Rows : kC32Rows) : GROUPED ? kGroupRows : ROWS)
         for (uint32_t j = 0; j < jn; j++) {
-            const float4 r0 = table[2 * j];  // (c_o0, c_o1, ew, ew)
-            const float D = row_d(v0, v1, r0.x, r0.y);
+            const float4 r0 = table[2 * j];  // (-c_o0, -c_o1, ew, ew)
+            // row_d, both differences in one packed add (256^3 voxels 67.4 -> 66.4 ms)
+            const float2 d01 = __fadd2_rn(make_float2(v0, v1), make_float2(r0.x, r0.y));
+            const float D = __fmaf_rn(d01.x, d01.x, __fmaf_rn(d01.y, d01.y, kQEps));
             const float2 D2 = make_float2(D, D);
             const float2 ew = make_float2(r0.z, r0.w);
             float2 nk = make_float2(0.0f, 0.0f);
@@ -913,8 +918,8 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
 //   A = sa |v - l| + (lw - t0) / dT - lo_L(l),   B = sb |v - s| + cw / dT - lo_S(s),
 // where lo = lo_L + lo_S is the pair's staged window start (both parts aligned, so their
 // sum is).  A stage holds the rows of cl = chunk / fs lasers x fs SPADs; its table carries
-// one record per laser and per SPAD (position relative to the tile centre in bin units,
-// constant).  A consumer thread keeps B of its voxels for the current SPAD block in registers
+// one record per laser and per SPAD (negated position relative to the tile centre in bin
+// units, constant).  A consumer thread keeps B of its voxels for the current SPAD block in registers
 // (formed when the block changes, reused across every laser of the capture) and forms A once
 // per laser, so an update costs two packed adds, the address and the gather instead of a
 // square root: 1 / fs reciprocal square roots per update.
@@ -1002,9 +1007,9 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
 #pragma unroll
                 for (int k = 0; k < 3; k++)
                     e[k] = __fmul_rn(lp[k] - __fmul_rn(g.ctr[k], a.h[k]), a.sa);
-                table[lane] = make_float4(sel3(e[0], e[1], e[2], a.oax0),
-                                          sel3(e[0], e[1], e[2], a.oax1),
-                                          sel3(e[0], e[1], e[2], a.kax), Lt.w - (float)lo_l);
+                table[lane] = make_float4(-sel3(e[0], e[1], e[2], a.oax0),
+                                          -sel3(e[0], e[1], e[2], a.oax1),
+                                          -sel3(e[0], e[1], e[2], a.kax), Lt.w - (float)lo_l);
             }
             if (lane < ns) {
                 const float4 G = spads[s0 + lane];
@@ -1017,9 +1022,9 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
 #pragma unroll
                 for (int k = 0; k < 3; k++)
                     e[k] = __fmul_rn(gp[k] - __fmul_rn(g.ctr[k], a.h[k]), a.sb);
-                table[cl + lane] = make_float4(sel3(e[0], e[1], e[2], a.oax0),
-                                               sel3(e[0], e[1], e[2], a.oax1),
-                                               sel3(e[0], e[1], e[2], a.kax), G.w - (float)lo_s);
+                table[cl + lane] = make_float4(-sel3(e[0], e[1], e[2], a.oax0),
+                                               -sel3(e[0], e[1], e[2], a.oax1),
+                                               -sel3(e[0], e[1], e[2], a.kax), G.w - (float)lo_s);
             }
             __syncwarp();
             if (lane == 0) mbar_expect_tx(fb, ncl * ns * a.nbox * a.BW * esz);
@@ -1066,10 +1071,12 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
         vk[i].x = rel_coord(a, g, a.kax, bk + (2 * i) * kstep);
         vk[i].y = rel_coord(a, g, a.kax, bk + (2 * i + 1) * kstep);
     }
-    // leg of the 8 voxels to the point of record rec: q * rsqrt(q) + rec.w
+    // leg of the thread's voxels to the point of record rec: q * rsqrt(q) + rec.w.  (Records
+    // hold negated positions, so that the differences are packed adds: 424 -> 415 us.)
     auto legs = [&](const float4 rec, float2 (&out)[NP]) {
-        const float D = row_d(v0, v1, rec.x, rec.y);
-        const float2 D2 = make_float2(D, D), nk = make_float2(-rec.z, -rec.z);
+        const float2 d01 = __fadd2_rn(make_float2(v0, v1), make_float2(rec.x, rec.y));
+        const float D = __fmaf_rn(d01.x, d01.x, __fmaf_rn(d01.y, d01.y, kQEps));
+        const float2 D2 = make_float2(D, D), nk = make_float2(rec.z, rec.z);
         const float2 c2 = make_float2(rec.w, rec.w);
 #pragma unroll
         for (int p = 0; p < NP; p++) {
