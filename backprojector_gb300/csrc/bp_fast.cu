@@ -1268,6 +1268,7 @@ __global__ void __launch_bounds__(288, CTAS)
     }
     PipeShared sh;
     pipeline_init(sh, smem_raw, full_bar, empty_bar, &abort_flag, a.stages);
+    allow_next();
     uint64_t step = 0;
     fast_unit<HT, K, KAHAN, CHECKED, PLANAR, kPlanRows, GROUPED>(a, &tmap, spads, lasers, dst,
                                                                  diag, t0, split, 0, step, sh);
@@ -1292,6 +1293,7 @@ __global__ void __launch_bounds__(288, fact_ctas(FORM))
     if (!plan_block<Pair<HT>>(a, out, block, tile, split, dst)) return;
     PipeShared sh;
     pipeline_init(sh, smem_raw, full_bar, empty_bar, &abort_flag, a.stages);
+    allow_next();
     uint64_t step = 0;
     fact_unit<HT, CHECKED, FORM>(a, &tmap, spads, lasers, dst, diag, tile, half, split, 0, step, sh);
     pipeline_drain(a.stages, step, full_bar, diag, a.spin_limit);
@@ -1365,6 +1367,7 @@ template <bool KAHAN>
 __global__ void __launch_bounds__(kReduceX *kReduceY)
     reduce_splits_kernel(const float *__restrict__ partial, float *__restrict__ out, uint64_t n,
                          uint32_t splits, float scale, int vec, int rows) {
+    wait_previous();
     const uint64_t quads = (n + 3) / 4;
     const bool vp = vec && n % 4 == 0;  // every split's block is 16-byte aligned
     if (KAHAN || !rows) {
@@ -1411,10 +1414,8 @@ void launch_reduce_splits(const float *partial, float *out, uint64_t n, uint32_t
     const unsigned blocks = (unsigned)((quads + per - 1) / per);
     const int vec = (uintptr_t)partial % 16 == 0 && (uintptr_t)out % 16 == 0;
     const dim3 threads(kReduceX, kReduceY);
-    if (kahan)
-        reduce_splits_kernel<true><<<blocks, threads, 0, s>>>(partial, out, n, splits, scale, vec, rows);
-    else
-        reduce_splits_kernel<false><<<blocks, threads, 0, s>>>(partial, out, n, splits, scale, vec, rows);
+    launch_after(kahan ? reduce_splits_kernel<true> : reduce_splits_kernel<false>, blocks, threads, 0,
+                 s, partial, out, n, splits, scale, vec, rows);
     count_launches(1);
 }
 
@@ -1427,6 +1428,7 @@ __global__ void __launch_bounds__(128)
     reduce_tiles_kernel(const float *__restrict__ partial, const uint32_t *__restrict__ list,
                         const uint32_t *__restrict__ count, uint32_t max_tiles, const FastArgs a,
                         float *__restrict__ out, int vec, const float *d_absmax, float target) {
+    wait_previous();
     const float factor = scale_of(1.0f, d_absmax, target);
     constexpr uint32_t C = COMPLEX ? 2 : 1;
     const uint32_t tz4 = a.tdim[2] * C / 4;  // tiles are a multiple of 4 voxels along z
@@ -2170,8 +2172,8 @@ int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const ui
         float *o = (float *)d_out;
         const int vec = (uintptr_t)d_out % 16 == 0 && (a.n[2] * (cplx ? 2 : 1)) % 4 == 0;
         auto run = [&](auto kernel) {
-            kernel<<<blocks, 128, 0, stream>>>(fp->d_partial, d_list, d_count, max_tiles, a, o, vec,
-                                                  d_absmax, target);
+            launch_after(kernel, blocks, 128, 0, stream, fp->d_partial, d_list, d_count, max_tiles, a,
+                         o, vec, d_absmax, target);
         };
         if (cplx)
             fp->kahan ? run(reduce_tiles_kernel<true, true>) : run(reduce_tiles_kernel<true, false>);

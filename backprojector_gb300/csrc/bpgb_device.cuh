@@ -74,6 +74,31 @@ __device__ __forceinline__ bool mbar_wait_backoff(uint32_t bar, uint32_t parity,
     return false;
 }
 
+// Programmatic dependent launch: a kernel queued by launch_after may become resident as soon as
+// every CTA of the kernel before it has called allow_next (or exited).  It must call
+// wait_previous, which returns once that kernel has completed and its writes are visible, in
+// every thread before it touches memory.  Both do nothing in ordinary launches.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, uint32_t smem,
+                         cudaStream_t stream, Args &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // 2-D tiled TMA load of a {box, 1} tile at (x, y) into shared memory, completing on bar.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int32_t x,
                                             int32_t y, uint32_t bar) {

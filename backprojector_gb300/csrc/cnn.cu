@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "bpgb_device.cuh"
 #include "bpgb_internal.h"
 
 namespace bpgb {
@@ -299,6 +300,8 @@ __global__ void bce_grad_kernel(const float *__restrict__ logits, const uint8_t 
 __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g,
                             float *__restrict__ m, float *__restrict__ v, uint64_t n, float lr,
                             float b1, float b2, float eps, float c1, float c2) {
+    wait_previous();
+    allow_next();
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const float gi = g[i];
@@ -569,8 +572,8 @@ int bpgb_cnn_adam(float *d_p, const float *d_g, float *d_m, float *d_v, uint64_t
     if (n == 0) return BPGB_OK;
     const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
     const unsigned grid = (unsigned)((n + 255) / 256 < 152 * 4 ? (n + 255) / 256 : 152 * 4);
-    adam_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_p, d_g, d_m, d_v, n, lr, beta1, beta2,
-                                                      eps, c1, c2);
+    launch_after(adam_kernel, grid, 256, 0, (cudaStream_t)stream, d_p, d_g, d_m, d_v, n, lr, beta1,
+                 beta2, eps, c1, c2);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;

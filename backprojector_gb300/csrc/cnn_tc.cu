@@ -147,6 +147,8 @@ __global__ void __launch_bounds__(kConvThreads)
     __shared__ __align__(8) uint64_t full[kConvStages], empty[kConvStages], acc_full[kConvAccs],
         acc_empty[kConvAccs], drain[2], wbar;
     __shared__ uint32_t taddr_s;
+    wait_previous();
+    allow_next();
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *w_s = smem;
     uint8_t *stage_s = smem + S::kWBytes;
@@ -403,6 +405,8 @@ __global__ void __launch_bounds__(kWgThreads)
     __shared__ __align__(8) uint64_t full[kWgStages], empty[kWgStages], done;
     __shared__ uint32_t taddr_s;
     __shared__ float bias_part[8][16];
+    wait_previous();
+    allow_next();
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *stage_s = smem;
 
@@ -573,6 +577,8 @@ __global__ void __launch_bounds__(256) wgrad_tc_reduce_kernel(const float *__res
                                                               uint32_t cin, uint32_t cout,
                                                               float *__restrict__ dW) {
     __shared__ float4 red[64][4];
+    wait_previous();
+    allow_next();
     const uint32_t k = blockIdx.x, q = threadIdx.x % 4, p0 = threadIdx.x / 4;
     float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (k <= 27 * cin)
@@ -608,6 +614,8 @@ __global__ void __launch_bounds__(256) wgrad_tc_reduce_kernel(const float *__res
 // Interior rows of an Lp tensor from channels-last BF16 [V][x_stride] (channels >= C zero).
 __global__ void lp_pack_kernel(const __nv_bfloat16 *__restrict__ X, uint32_t C, uint32_t xs, Lp g,
                                uint8_t *__restrict__ out) {
+    wait_previous();
+    allow_next();
     const uint64_t n = (uint64_t)g.batch * g.n0 * g.n1 * 32 * g.npl;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -683,6 +691,8 @@ struct PackJobs {
 };
 
 __global__ void pack_tc_jobs_kernel(PackJobs p) {
+    wait_previous();
+    allow_next();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= p.start[p.jobs]) return;
     uint32_t j = 0;
@@ -711,6 +721,8 @@ __global__ void pack_tc_jobs_kernel(PackJobs p) {
 __global__ void bce_lp_kernel(const float *__restrict__ logits, const uint8_t *__restrict__ y,
                               Lp g, float pos_weight, float scale, uint8_t *__restrict__ dZ,
                               float *__restrict__ loss) {
+    wait_previous();
+    allow_next();
     const uint64_t n = (uint64_t)g.batch * g.n0 * g.n1 * 32;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -789,7 +801,7 @@ int bpgb_cnn_lp_pack(const void *d_X, uint32_t channels, uint32_t x_stride, cons
         return set_error(BPGB_ERR_INVALID_ARGUMENT,
                          "bad lp_pack arguments (dims[2] must be 32, dims[1] a multiple of 8)");
     const uint64_t n = (uint64_t)batch * g.n0 * g.n1 * 32 * g.npl;
-    lp_pack_kernel<<<grid_for(n, 256, 152 * 16), 256, 0, (cudaStream_t)stream>>>(
+    launch_after(lp_pack_kernel, grid_for(n, 256, 152 * 16), 256, 0, (cudaStream_t)stream,
         (const __nv_bfloat16 *)d_X, channels, x_stride, g, (uint8_t *)d_lp);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
@@ -856,7 +868,7 @@ int bpgb_cnn_tc_pack_layers(const float *const *d_W, const uint32_t *cin, const 
     }
     p.jobs = 2 * layers;
     p.start[p.jobs] = n;
-    pack_tc_jobs_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(p);
+    launch_after(pack_tc_jobs_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, p);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;
@@ -906,7 +918,7 @@ int bpgb_cnn_tc_conv3d(const void *d_X, uint32_t in_channels, uint32_t in_zpad,
         smem = std::max(kMinSmem, smem);
         if ((st = reserve_dynamic_smem((const void *)kernel, smem))) return st;
         const unsigned grid = (unsigned)std::min<uint64_t>(a.nblocks, 2ull * sm_count_cached());
-        kernel<<<grid, kConvThreads, smem, s>>>(map, a);
+        launch_after(kernel, grid, kConvThreads, smem, s, map, a);
         return BPGB_OK;
     };
     st = a.in.npl == 2 ? launch(conv_tc_kernel<2>, ConvShape<2>::kSmem)
@@ -995,15 +1007,15 @@ int bpgb_cnn_tc_conv3d_wgrad(const void *d_X, uint32_t in_channels, const void *
     auto launch = [&](auto kernel, uint32_t smem) -> int {
         smem = std::max(kMinSmem, smem);
         if ((st = reserve_dynamic_smem((const void *)kernel, smem))) return st;
-        kernel<<<grid, kWgThreads, smem, s>>>(xmap, map, a);
+        launch_after(kernel, grid, kWgThreads, smem, s, xmap, map, a);
         return BPGB_OK;
     };
     st = a.xin.npl == 2 ? launch(wgrad_tc_kernel<2>, WgShape<2>::kSmem)
                         : launch(wgrad_tc_kernel<1>, WgShape<1>::kSmem);
     if (st) return st;
     count_launches(1);
-    wgrad_tc_reduce_kernel<<<a.kp, 256, 0, s>>>(d_scratch, grid, a.kp, in_channels, out_channels,
-                                                d_dW);
+    launch_after(wgrad_tc_reduce_kernel, a.kp, 256, 0, s, d_scratch, grid, a.kp, in_channels,
+                 out_channels, d_dW);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;
@@ -1017,7 +1029,7 @@ int bpgb_cnn_tc_bce_grad(const float *d_logits, const uint8_t *d_labels, const u
     if (!d_logits || !d_labels || !d_dZ || !lp_of(dims, batch, 1, 1, &g) || !aligned16(d_dZ))
         return set_error(BPGB_ERR_INVALID_ARGUMENT, "bad tc_bce_grad arguments");
     const uint64_t n = (uint64_t)batch * g.n0 * g.n1 * 32;
-    bce_lp_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, (cudaStream_t)stream>>>(
+    launch_after(bce_lp_kernel, grid_for(n, 256, 152 * 8), 256, 0, (cudaStream_t)stream,
         d_logits, d_labels, g, pos_weight, scale, (uint8_t *)d_dZ, d_loss);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
