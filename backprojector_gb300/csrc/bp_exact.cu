@@ -144,6 +144,8 @@ __global__ void __launch_bounds__(kThreads)
     bp_exact_kernel(const HT *__restrict__ H, const bpgb_pair *__restrict__ pairs,
                     HT *__restrict__ out, const ExactArgs a) {
     constexpr int NP = kTX / 2;
+    wait_previous();
+    allow_next();
     __shared__ Staged sp[2][kGroup];
     uint32_t t = blockIdx.x / a.splits;
     const uint32_t z = t % a.tiles[2] * kTZ + threadIdx.x % kTZ;
@@ -251,6 +253,8 @@ __global__ void __launch_bounds__(kThreads)
 template <typename HT>
 __global__ void exact_reduce_kernel(const HT *__restrict__ partial, HT *__restrict__ out,
                                     uint64_t nvox, uint32_t splits) {
+    wait_previous();
+    allow_next();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= nvox) return;
     HT v[kMaxSplits];
@@ -393,17 +397,16 @@ int launch_exact(const void *d_H, bool is_complex, uint64_t pitch, const bpgb_pa
                                              : (void *)bp_exact_kernel<float2, false>)
                             : (filter.inside ? (void *)bp_exact_kernel<float, true>
                                              : (void *)bp_exact_kernel<float, false>);
-    BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3((unsigned)(tiles * splits)), dim3(kThreads), args, 0,
-                                   stream));
+    BPGB_CUDA_TRY(launch_after(kern, (unsigned)(tiles * splits), kThreads, args, 0, stream));
     count_launches(1);
     if (splits > 1) {
         const unsigned blocks = (unsigned)((a.nvox + 255) / 256);
         if (is_complex)
-            exact_reduce_kernel<float2><<<blocks, 256, 0, stream>>>(
-                (const float2 *)d_partial, (float2 *)d_out, a.nvox, splits);
+            launch_after(exact_reduce_kernel<float2>, blocks, 256, 0, stream,
+                         (const float2 *)d_partial, (float2 *)d_out, a.nvox, splits);
         else
-            exact_reduce_kernel<float><<<blocks, 256, 0, stream>>>(
-                (const float *)d_partial, (float *)d_out, a.nvox, splits);
+            launch_after(exact_reduce_kernel<float>, blocks, 256, 0, stream, (const float *)d_partial,
+                         (float *)d_out, a.nvox, splits);
         count_launches(1);
         BPGB_CUDA_TRY(cudaGetLastError());
     }

@@ -1261,6 +1261,7 @@ __global__ void __launch_bounds__(288, CTAS)
     __shared__ int abort_flag;
     uint32_t t0, split;
     void *dst = out;
+    if (a.tile_list) wait_previous();  // the list may be the kernel before's
     if constexpr (GROUPED) {
         if (!plan_group<Pair<HT>>(a, out, t0, split)) return;
     } else {
@@ -1268,6 +1269,7 @@ __global__ void __launch_bounds__(288, CTAS)
     }
     PipeShared sh;
     pipeline_init(sh, smem_raw, full_bar, empty_bar, &abort_flag, a.stages);
+    wait_previous();
     allow_next();
     uint64_t step = 0;
     fast_unit<HT, K, KAHAN, CHECKED, PLANAR, kPlanRows, GROUPED>(a, &tmap, spads, lasers, dst,
@@ -1290,9 +1292,11 @@ __global__ void __launch_bounds__(288, fact_ctas(FORM))
     void *dst;
     const uint32_t half = FORM == FACT_HALF ? blockIdx.x & 1 : 0;
     const uint32_t block = FORM == FACT_HALF ? blockIdx.x / 2 : blockIdx.x;
+    if (a.tile_list) wait_previous();  // the list may be the kernel before's
     if (!plan_block<Pair<HT>>(a, out, block, tile, split, dst)) return;
     PipeShared sh;
     pipeline_init(sh, smem_raw, full_bar, empty_bar, &abort_flag, a.stages);
+    wait_previous();
     allow_next();
     uint64_t step = 0;
     fact_unit<HT, CHECKED, FORM>(a, &tmap, spads, lasers, dst, diag, tile, half, split, 0, step, sh);
@@ -1368,6 +1372,7 @@ __global__ void __launch_bounds__(kReduceX *kReduceY)
     reduce_splits_kernel(const float *__restrict__ partial, float *__restrict__ out, uint64_t n,
                          uint32_t splits, float scale, int vec, int rows) {
     wait_previous();
+    allow_next();
     const uint64_t quads = (n + 3) / 4;
     const bool vp = vec && n % 4 == 0;  // every split's block is 16-byte aligned
     if (KAHAN || !rows) {
@@ -1429,6 +1434,7 @@ __global__ void __launch_bounds__(128)
                         const uint32_t *__restrict__ count, uint32_t max_tiles, const FastArgs a,
                         float *__restrict__ out, int vec, const float *d_absmax, float target) {
     wait_previous();
+    allow_next();
     const float factor = scale_of(1.0f, d_absmax, target);
     constexpr uint32_t C = COMPLEX ? 2 : 1;
     const uint32_t tz4 = a.tdim[2] * C / 4;  // tiles are a multiple of 4 voxels along z
@@ -2123,7 +2129,7 @@ int fast_plan_execute(FastPlan *fp, const void *d_H, void *d_out, cudaStream_t s
     unsigned long long *diag = fp->d_diag;
     void *args[] = {(void *)&map, (void *)&spads, (void *)&lasers, (void *)&target,
                     (void *)&diag, (void *)&fp->a};
-    BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3(fp->grid), dim3(fp->threads), args, fp->smem, stream));
+    BPGB_CUDA_TRY(launch_after(kern, fp->grid, fp->threads, args, fp->smem, stream));
     count_launches(1);
     if (a.splits > 1) {
         const bool cplx = fp->dtype == BPGB_DTYPE_C64 || fp->dtype == BPGB_DTYPE_C32;
@@ -2163,8 +2169,8 @@ int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const ui
     void *kern = plan_kernel(fp);
     void *args[] = {(void *)&map, (void *)&spads, (void *)&lasers, (void *)&dst,
                     (void *)&fp->d_diag, (void *)&a};
-    BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3((uint32_t)(slot_groups * a.splits)),
-                                   dim3(fp->threads), args, fp->smem, stream));
+    BPGB_CUDA_TRY(launch_after(kern, (uint32_t)(slot_groups * a.splits), fp->threads, args, fp->smem,
+                               stream));
     count_launches(1);
     if (a.splits > 1) {
         const bool cplx = fp->dtype == BPGB_DTYPE_C64 || fp->dtype == BPGB_DTYPE_C32;
@@ -3154,7 +3160,7 @@ extern "C" int bpgb_backproject_noalloc(const float *d_H, uint32_t T, uint32_t h
     const float4 *lasers = tab + num_spads;
     void *args[] = {(void *)&map, (void *)&spads, (void *)&lasers, (void *)&target, (void *)&diag,
                     (void *)&a};
-    BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3((unsigned)(ntiles * splits)), dim3(threads), args, smem, s));
+    BPGB_CUDA_TRY(launch_after(kern, (unsigned)(ntiles * splits), threads, args, smem, s));
     count_launches(1);
     if (a.splits > 1) {
         launch_reduce_splits(partial, d_volume, a.nvox, a.splits, 1.0f, false, s);

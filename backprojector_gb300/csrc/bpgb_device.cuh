@@ -83,20 +83,31 @@ __device__ __forceinline__ void allow_next() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <typename... Params, typename... Args>
-cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, uint32_t smem,
-                         cudaStream_t stream, Args &&...args) {
+inline cudaLaunchConfig_t after_config(cudaLaunchAttribute *attr, dim3 grid, dim3 block,
+                                       uint32_t smem, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    return cfg;
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, uint32_t smem,
+                         cudaStream_t stream, Args &&...args) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = after_config(&attr, grid, block, smem, stream);
     return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+inline cudaError_t launch_after(const void *kernel, dim3 grid, dim3 block, void **args,
+                                uint32_t smem, cudaStream_t stream) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = after_config(&attr, grid, block, smem, stream);
+    return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 // 2-D tiled TMA load of a {box, 1} tile at (x, y) into shared memory, completing on bar.

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(256)
     upsample_kernel(const float *__restrict__ coarse, uint32_t c0, uint32_t c1, uint32_t c2,
                     float *__restrict__ fine, uint32_t f0, uint32_t f1, uint32_t f2, uint32_t lines,
                     int vec, const float *d_absmax, float target) {
+    wait_previous();
+    allow_next();
     const float factor = scale_of(1.0f, d_absmax, target);
     extern __shared__ float line[];  // lines x c2 floats
     const uint32_t j0 = blockIdx.x * lines, i = blockIdx.y;
@@ -280,7 +282,7 @@ int upsample_scaled(const float *d_coarse, const uint32_t *coarse_dims, float *d
     const uint32_t lines = std::min<uint32_t>(8, 12288 / coarse_dims[2]);
     const dim3 grid((fine_dims[1] + lines - 1) / lines, fine_dims[0]);
     const int vec = fine_dims[2] % 4 == 0 && (uintptr_t)d_fine % 16 == 0;
-    upsample_kernel<<<grid, 256, lines * coarse_dims[2] * sizeof(float), stream>>>(
+    launch_after(upsample_kernel, grid, 256, (uint32_t)(lines * coarse_dims[2] * sizeof(float)), stream,
         d_coarse, coarse_dims[0], coarse_dims[1], coarse_dims[2], d_fine, fine_dims[0],
         fine_dims[1], fine_dims[2], lines, vec, d_absmax, target);
     count_launches(1);

@@ -23,6 +23,7 @@
 #include <mutex>
 #include <vector>
 
+#include "bpgb_device.cuh"
 #include "bpgb_internal.h"
 
 namespace bpgb {
@@ -63,6 +64,8 @@ __global__ void __launch_bounds__(kMaxThreads)
                         const float2 *__restrict__ taps, int K, float2 *__restrict__ out,
                         uint32_t out_pitch, uint32_t nseg, int vec) {
     extern __shared__ __align__(16) float sm[];
+    wait_previous();
+    allow_next();
     const int groups = blockDim.x + (min(K, kTapBlock) + kPer - 1) / kPer + 2;
     float4 *tp4 = reinterpret_cast<float4 *>(sm + (size_t)groups * kGroupWords);
     float2 *tp = reinterpret_cast<float2 *>(tp4);
@@ -185,8 +188,8 @@ int launch_phasor_pulse(const float *d_H, uint64_t rows, uint32_t T, uint32_t in
     if (int rs = reserve_dynamic_smem((const void *)phasor_pulse_kernel, p.smem)) return rs;
     // 16-byte stores where every row's outputs are 16-byte aligned
     const int vec = ((uintptr_t)d_out % 16 == 0 && out_pitch % 2 == 0) ? 1 : 0;
-    phasor_pulse_kernel<<<(unsigned)blocks, p.threads, p.smem, stream>>>(
-        d_H, T, in_pitch, d_taps, K, reinterpret_cast<float2 *>(d_out), out_pitch, p.nseg, vec);
+    launch_after(phasor_pulse_kernel, (unsigned)blocks, p.threads, p.smem, stream, d_H, T, in_pitch,
+                 d_taps, K, reinterpret_cast<float2 *>(d_out), out_pitch, p.nseg, vec);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;

@@ -40,6 +40,8 @@ unsigned blocks_for(const Rows &g) {
 template <bool VEC>
 __global__ void __launch_bounds__(256)
     absmax_kernel(const float *__restrict__ in, const Rows g, unsigned int *__restrict__ out) {
+    wait_previous();
+    allow_next();
     unsigned int m = 0;
     auto take = [&](float v) { m = max(m, __float_as_uint(v) & 0x7fffffffu); };
     for (uint64_t q = blockIdx.x; q < g.rows * g.pieces; q += gridDim.x) {
@@ -86,6 +88,8 @@ template <typename HT, bool VEC>
 __global__ void __launch_bounds__(256)
     to_half_kernel(const float *__restrict__ in, const Rows g, uint64_t T, float scale,
                    const float *__restrict__ d_absmax, float target, HT *__restrict__ out) {
+    wait_previous();
+    allow_next();
     const float inv_scale = 1.0f / scale_of(scale, d_absmax, target);
     const uint64_t count = g.rows * g.pieces;
     for (uint64_t b = blockIdx.x; b < count; b += gridDim.x) {
@@ -130,6 +134,8 @@ template <bool VEC>
 __global__ void __launch_bounds__(256)
     scale_kernel(float *__restrict__ v, uint64_t n, float scale,
                  const float *__restrict__ d_absmax, float target) {
+    wait_previous();
+    allow_next();
     const float f = scale_of(scale, d_absmax, target);
     const uint64_t step = (uint64_t)gridDim.x * 256, at = blockIdx.x * 256ull + threadIdx.x;
     uint64_t i = at;
@@ -166,9 +172,9 @@ int bpgb_rows_absmax(const float *d_H, uint64_t rows, uint32_t T, uint32_t pitch
     if (n == 0) return BPGB_OK;
     const Rows g = rows_of(rows, T, pitch, pitch == T);
     if (aligned16(d_H) && (g.rows == 1 || pitch % 4 == 0))
-        absmax_kernel<true><<<blocks_for(g), 256, 0, s>>>(d_H, g, (unsigned int *)d_max);
+        launch_after(absmax_kernel<true>, blocks_for(g), 256, 0, s, d_H, g, (unsigned int *)d_max);
     else
-        absmax_kernel<false><<<blocks_for(g), 256, 0, s>>>(d_H, g, (unsigned int *)d_max);
+        launch_after(absmax_kernel<false>, blocks_for(g), 256, 0, s, d_H, g, (unsigned int *)d_max);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;
@@ -190,7 +196,8 @@ int bpgb_rows_to_half(const float *d_H, uint64_t rows, uint32_t T, uint32_t in_p
     const bool vec = aligned16(d_H) && aligned16(d_out) &&
                      (g.rows == 1 || (in_pitch % 4 == 0 && out_pitch % 8 == 0));
     auto run = [&](auto kernel, auto *out) {
-        kernel<<<blocks_for(g), 256, 0, s>>>(d_H, g, flat ? g.T : T, scale, d_absmax, target, out);
+        launch_after(kernel, blocks_for(g), 256, 0, s, d_H, g, flat ? g.T : T, scale, d_absmax, target,
+                     out);
     };
     if (dtype == BPGB_DTYPE_F16)
         vec ? run(to_half_kernel<__half, true>, (__half *)d_out)
@@ -213,9 +220,9 @@ int bpgb_volume_scale(float *d_volume, uint64_t n, float scale, const float *d_a
     const unsigned grid = (unsigned)(want < 152 * 16 ? want : 152 * 16);
     cudaStream_t s = (cudaStream_t)stream;
     if (aligned16(d_volume))
-        scale_kernel<true><<<grid, 256, 0, s>>>(d_volume, n, scale, d_absmax, target);
+        launch_after(scale_kernel<true>, grid, 256, 0, s, d_volume, n, scale, d_absmax, target);
     else
-        scale_kernel<false><<<grid, 256, 0, s>>>(d_volume, n, scale, d_absmax, target);
+        launch_after(scale_kernel<false>, grid, 256, 0, s, d_volume, n, scale, d_absmax, target);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
     return BPGB_OK;
