@@ -124,6 +124,7 @@ struct FastArgs {
     // tile-list launches with pair splits: partial sums are stored per list slot and
     // split at tile-local voxel offsets (slot-major, then split, then voxel)
     uint32_t tile_local;
+    uint32_t block0;  // first CTA of a launch over some of the pair splits
     // lasers x SPADs with factored legs (bp_fact_kernel): fs SPADs per block (0: per-pair
     // legs); nchunks then counts laser groups
     uint32_t fs;
@@ -1265,7 +1266,7 @@ __global__ void __launch_bounds__(288, CTAS)
     if constexpr (GROUPED) {
         if (!plan_group<Pair<HT>>(a, out, t0, split)) return;
     } else {
-        if (!plan_block<Pair<HT>>(a, out, blockIdx.x, t0, split, dst)) return;
+        if (!plan_block<Pair<HT>>(a, out, a.block0 + blockIdx.x, t0, split, dst)) return;
     }
     PipeShared sh;
     pipeline_init(sh, smem_raw, full_bar, empty_bar, &abort_flag, a.stages);
@@ -2116,28 +2117,73 @@ int fast_plan_build(FastPlan **out, const bpgb_pair *d_pairs, uint64_t P,
     return BPGB_OK;
 }
 
-int fast_plan_execute(FastPlan *fp, const void *d_H, void *d_out, cudaStream_t stream) {
-    const FastArgs &a = fp->a;
+namespace {
+
+// The plan's CTAs of pair splits [s0, s1) on `stream`; after_previous: as launch_after.
+int launch_splits(FastPlan *fp, const void *d_H, void *d_out, uint32_t s0, uint32_t s1,
+                  bool after_previous, cudaStream_t stream) {
+    FastArgs a = fp->a;
     if (((uintptr_t)d_H) % 16) return set_error(BPGB_ERR_INVALID_ARGUMENT, "H must be 16-byte aligned");
     CUtensorMap map;
     int st = encode_rows(&map, fp->dtype, d_H, a.T, fp->P, fp->pitch, a.BW);
     if (st) return st;
+    const uint32_t per_split = fp->grid / a.splits;
+    a.block0 = per_split * s0;
     void *target = a.splits > 1 ? (void *)fp->d_partial : d_out;
     const float4 *spads = fp->d_tables;
     const float4 *lasers = fp->d_tables + a.S;
     void *kern = plan_kernel(fp);
     unsigned long long *diag = fp->d_diag;
     void *args[] = {(void *)&map, (void *)&spads, (void *)&lasers, (void *)&target,
-                    (void *)&diag, (void *)&fp->a};
-    BPGB_CUDA_TRY(launch_after(kern, fp->grid, fp->threads, args, fp->smem, stream));
+                    (void *)&diag, (void *)&a};
+    const uint32_t grid = per_split * (s1 - s0);
+    if (after_previous)
+        BPGB_CUDA_TRY(launch_after(kern, grid, fp->threads, args, fp->smem, stream));
+    else
+        BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3(grid), dim3(fp->threads), args, fp->smem, stream));
     count_launches(1);
-    if (a.splits > 1) {
-        const bool cplx = fp->dtype == BPGB_DTYPE_C64 || fp->dtype == BPGB_DTYPE_C32;
-        launch_reduce_splits(fp->d_partial, (float *)d_out, a.nvox * (cplx ? 2 : 1), a.splits,
-                             a.out_scale, fp->kahan, stream);
-        BPGB_CUDA_TRY(cudaGetLastError());
-    }
     return BPGB_OK;
+}
+
+int reduce_plan(FastPlan *fp, void *d_out, cudaStream_t stream) {
+    const FastArgs &a = fp->a;
+    if (a.splits == 1) return BPGB_OK;
+    const bool cplx = fp->dtype == BPGB_DTYPE_C64 || fp->dtype == BPGB_DTYPE_C32;
+    launch_reduce_splits(fp->d_partial, (float *)d_out, a.nvox * (cplx ? 2 : 1), a.splits, a.out_scale,
+                         fp->kahan, stream);
+    BPGB_CUDA_TRY(cudaGetLastError());
+    return BPGB_OK;
+}
+
+}  // namespace
+
+int fast_plan_execute(FastPlan *fp, const void *d_H, void *d_out, cudaStream_t stream) {
+    const int st = launch_splits(fp, d_H, d_out, 0, fp->a.splits, true, stream);
+    return st ? st : reduce_plan(fp, d_out, stream);
+}
+
+uint32_t fast_plan_parts(const FastPlan *fp) {
+    // Rows are used in their order by per-pair legs with one tile per CTA; the factored form
+    // takes every laser's rows of a SPAD block, and the grouped form numbers its CTAs otherwise.
+    return fp->fact || fp->grouped ? 1 : std::min<uint32_t>(fp->a.splits, kMaxParts);
+}
+
+uint64_t fast_plan_part_rows(const FastPlan *fp, uint32_t part, uint32_t parts) {
+    const FastArgs &a = fp->a;
+    const uint64_t items = fast_items(a), s1 = (uint64_t)a.splits * (part + 1) / parts;
+    const uint64_t i1 = items * s1 / a.splits;  // the first item after the part's last split
+    return i1 / a.nchunks * a.S + std::min<uint64_t>(a.S, i1 % a.nchunks * a.chunk);
+}
+
+int fast_plan_execute_part(FastPlan *fp, const void *d_H, void *d_out, uint32_t part, uint32_t parts,
+                           cudaStream_t stream) {
+    const uint32_t n = fp->a.splits;
+    return launch_splits(fp, d_H, d_out, (uint32_t)((uint64_t)n * part / parts),
+                         (uint32_t)((uint64_t)n * (part + 1) / parts), false, stream);
+}
+
+int fast_plan_reduce(FastPlan *fp, void *d_out, cudaStream_t stream) {
+    return reduce_plan(fp, d_out, stream);
 }
 
 int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const uint32_t *d_list,

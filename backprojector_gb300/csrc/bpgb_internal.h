@@ -121,6 +121,15 @@ int fast_plan_build(FastPlan **out, const bpgb_pair *d_pairs, uint64_t P,
                     const Factorization &fz, const Volume &vol, const BinParams &bp,
                     const bpgb_options &opt, int sm_count, std::string *why_not);
 int fast_plan_execute(FastPlan *fp, const void *d_H, void *d_out, cudaStream_t stream);
+// A plan's pass in `parts` launches over consecutive pair splits (and so, in these plans, over
+// consecutive rows of H), which may run as the rows arrive: part k needs the first
+// fast_plan_part_rows(k) rows; fast_plan_reduce follows all of them.
+constexpr uint32_t kMaxParts = 4;
+uint32_t fast_plan_parts(const FastPlan *fp);  // the most that make sense (1: run it whole)
+uint64_t fast_plan_part_rows(const FastPlan *fp, uint32_t part, uint32_t parts);
+int fast_plan_execute_part(FastPlan *fp, const void *d_H, void *d_out, uint32_t part, uint32_t parts,
+                           cudaStream_t stream);
+int fast_plan_reduce(FastPlan *fp, void *d_out, cudaStream_t stream);
 int fast_plan_dump_bins(FastPlan *fp, const int64_t *d_ids, int64_t n, int32_t *d_bins,
                         cudaStream_t stream);
 int fast_plan_execute_tiles(FastPlan *fp, const void *d_H, void *d_out, const uint32_t *d_list,

@@ -121,3 +121,32 @@ def test_conversion_chain(cuda):
         got = [one(1.0 + k, False) for k in range(20)]
         torch.cuda.synchronize()
         assert all(torch.equal(g, one(1.0 + k, True)) for k, g in enumerate(got))
+
+
+@pytest.mark.parametrize("T,spads,lasers,opt", [
+    (1100, (32, 33), None, {}), (1101, (32, 33), None, {"pair_splits": 3}),
+    (2051, (29, 18), None, {"pair_splits": 9, "chunk": 7}),
+    (1100, (10, 9), (4, 3), {"unfactored": 1, "pair_splits": 5}),
+    (1100, (12, 10), (4, 3), {}), (1100, (32, 33), None, {"accum": capi.ACCUM_KAHAN}),
+    (1100, (32, 33), None, {"pair_splits": 1}), (1100, (32, 33), None, {"algo": capi.ALGO_EXACT}),
+])
+def test_host_call_in_parts_equals_a_plan(cuda, T, spads, lasers, opt):
+    """Captures large enough to be uploaded in parts: the host call's volume is the plan's, bit
+    for bit, on the first call and on repeats with new rows."""
+    import torch
+
+    c = synthetic.make_capture("precision_64" if lasers is None else "dense_exhaustive_16", seed=1,
+                               render=False, spad_grid=spads, laser_grid=lasers, T=T, deltaT=0.003)
+    n, rng = (21, 18, 23), np.random.default_rng(T)
+    zero, inc = capi.volume_basis(c.volume_position, c.volume_size, np.uint32(n))
+    pitch = (T + 3) // 4 * 4
+    assert c.P * T * 4 >= 4 << 20
+    rows, V = torch.zeros((c.P, pitch), device=cuda), torch.empty(n, device=cuda)
+    with capi.Plan(c.pairs, T, n, zero, inc, c.t0, c.deltaT, h_pitch=pitch, **opt) as plan:
+        for _ in range(3):
+            H = rng.random((c.P, T), dtype=np.float32)
+            rows[:, :T] = torch.from_numpy(H).to(cuda)
+            plan.execute(rows, V)
+            want = V.cpu().numpy()
+            got = capi.backproject_host(H, c.pairs, n, zero, inc, c.t0, c.deltaT, **opt)
+            assert np.array_equal(got, want)
