@@ -81,7 +81,8 @@ __host__ __device__ constexpr uint32_t table_bytes_of(uint32_t c) {
     return (c * kRecordBytes + 127) / 128 * 128;
 }
 // shared memory of a CTA's stages when three CTAs of 8 consumer warps share an SM
-constexpr uint32_t kWideSoft = 72 * 1024;
+constexpr uint32_t kWideSoft = 74 * 1024;
+constexpr uint32_t kFillSoft = 72 * 1024;  // the same for pair_splits < 0, whose sums stay put
 constexpr float kMargin = 2.0f;                            // bins of slack around each window
 constexpr float kQEps = 1e-6f;                             // keeps q > 0 (bins^2)
 
@@ -827,8 +828,9 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
         // 3.47 ms, 8 rows 3.32, 16 rows 3.38; the batch kernel 4 rows 36.96, 8 rows 36.74, 16 rows
         // 36.91; complex64 rows (128^3) 1 row 16.14, 2 rows 16.08.
         const uint32_t jn = live ? nrows : 0u;  // a tile past the list or volume idles
-#pragma unroll(PairT::kCplx ? (PairT::kEsz == 8 ? kC64Rows : kC32Rows) : GROUPED ? kGroupRows : ROWS)
-        for (uint32_t j = 0; j < jn; j++) {
+        constexpr uint32_t kRows = PairT::kCplx ? (PairT::kEsz == 8 ? kC64Rows : kC32Rows)
+                                                : GROUPED ? kGroupRows : ROWS;
+        auto rows_at = [&](uint32_t j) {
             const float4 r0 = table[2 * j];  // (-c_o0, -c_o1, ew, ew)
             // row_d, both differences in one packed add (256^3 voxels 67.4 -> 66.4 ms)
             const float2 d01 = __fadd2_rn(make_float2(v0, v1), make_float2(r0.x, r0.y));
@@ -870,7 +872,25 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
                 else
                     acc[p].gather2(at.x, at.y);
             }
+        };
+        uint32_t j = 0;
+#pragma unroll 1
+        for (; j + kRows <= jn; j += kRows) {
+#pragma unroll
+            for (uint32_t u = 0; u < kRows; u++) rows_at(j + u);
         }
+        if (kRows > 8 && jn - j >= 8) {
+#pragma unroll
+            for (uint32_t u = 0; u < 8; u++) rows_at(j + u);
+            j += 8;
+        }
+        if (kRows > 4 && jn - j >= 4) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) rows_at(j + u);
+            j += 4;
+        }
+#pragma unroll 1
+        for (; j < jn; j++) rows_at(j);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_addr(&empty_bar[stage]));
         if (KAHAN) {
@@ -1781,9 +1801,12 @@ void *select_fact_kernel(int dtype, bool checked, bool half) {
     return nullptr;
 }
 
-// The next smaller default stage: whole unrolled iterations of kPlanRows rows, then halves.
+// The next smaller default stage, in the row counts that the consumers' unrolled bodies divide:
+// multiples of 16, then of 8, then of 4 (64^3 voxels, 384-bin windows: 8 rows 335 us, 12 rows
+// 316, 16 rows 303, 24 rows 297).
 uint32_t fewer_rows(uint32_t chunk) {
-    return chunk > 16 ? (chunk - 1) / kPlanRows * kPlanRows : (chunk + 1) / 2;
+    const uint32_t step = chunk > 32 ? 16 : chunk > 16 ? 8 : 4;
+    return chunk > 8 ? (chunk - 1) / step * step : (chunk + 1) / 2;
 }
 
 // Launch arguments of the fast kernel for a volume, pair factorisation and tile preset:
@@ -1866,7 +1889,7 @@ int fast_args(FastArgs &a, const FastConfig &cfg, const Volume &vol, const doubl
                                  : (cwarps == 4 ? 4 : 7);
     const uint32_t soft = ctas >= 7   ? 38 * 1024
                           : ctas >= 4 ? 56 * 1024
-                          : ctas >= 3 ? kWideSoft
+                          : ctas >= 3 ? (halve ? kFillSoft : kWideSoft)
                           : (ctas == 2 ? 110 * 1024 : 200 * 1024);
     const uint32_t budget = 200 * 1024;
     // Long chunks amortise the per-stage handshake (measured: 8 -> 32 rows cut the

@@ -100,3 +100,39 @@ def test_upsample_edges(cuda, coarse, fine):
         ref = np.take(ref, lo, a) * (1 - w) + np.take(ref, hi, a) * w
     # FP32 weights are within a few 1e-6 (grid coordinates up to 9), values of order 1
     np.testing.assert_allclose(out.cpu().numpy(), ref, atol=2e-5)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "c64", "c32"])
+@pytest.mark.parametrize("tile", [-1, 13])
+def test_rows_per_stage(cuda, dtype, tile):
+    """Stages of every remainder of the unrolled rows (16, 8, 4, 1) give one volume: integer
+    rows, small enough to be exact in 16 bits."""
+    import torch
+
+    if tile == 13 and dtype[0] == "c":
+        pytest.skip("several tiles per CTA: real rows")
+    c = synthetic.make_capture("precision_64", seed=5, render=False, spad_grid=(11, 9), T=512,
+                               deltaT=0.007)
+    rng = np.random.default_rng(3)
+    H = torch.from_numpy(rng.integers(0, 100, (c.P, c.T)).astype(np.float32)).to(cuda)
+    if dtype == "c64":
+        rows = torch.complex(H, H.flip(1))
+    elif dtype == "c32":
+        rows = torch.stack([H, H.flip(1)], -1).half().contiguous()
+    else:
+        rows = H.bfloat16() if dtype == "bf16" else H
+    n = (18, 11, 19)
+    zero, inc = capi.volume_basis(c.volume_position, c.volume_size, np.uint32(n))
+    code = {"f32": capi.DTYPE_F32, "bf16": capi.DTYPE_BF16, "c64": capi.DTYPE_C64,
+            "c32": capi.DTYPE_C32}[dtype]
+    want = None
+    for chunk in (1, 2, 3, 4, 5, 7, 8, 11, 12, 15, 16, 17, 20, 24, 29, 31, 32, 47, 64):
+        V = torch.full(n, float("nan"), dtype=torch.complex64 if dtype[0] == "c" else torch.float32,
+                       device=cuda)
+        with capi.Plan(c.pairs, c.T, n, zero, inc, c.t0, c.deltaT, algo=capi.ALGO_FAST, h_dtype=code,
+                       chunk=chunk, tile=tile) as p:
+            p.execute(rows, V)
+            p.check()
+        got = V.cpu().numpy()
+        want = got if want is None else want
+        assert np.array_equal(got, want), chunk
