@@ -22,16 +22,17 @@
 // its lanes.  E = 0.5 (scales where the bound does not hold) marks every update.
 //
 // Bound: issue (24 instructions per update, the marked ones' evaluations included) and the
-// latency of the L1 gathers.  Measured on 64 x 64 pairs that do
-// not factor, T = 2048, 64^3 voxels: 3.60 ms before, 0.97 ms with the filter.
+// latency of the L1 gathers.  Measured on 64 x 64 pairs that do not factor, T = 2048, 64^3
+// voxels: 3.60 ms before, 0.95 ms with the filter.
 //
-// Layout: one CTA = 64 threads = a 4 x 8 x 8 voxel tile (z fastest, x slowest), the four
-// voxels of an x line per thread as two packed FP32x2 lane pairs.  Pair records are staged 64 at a
-// time in shared memory, coordinates doubled for the packed arithmetic, and read as
-// warp-uniform broadcasts; a warp's 128 voxels gather from one H row at neighbouring bins,
-// so the global gathers coalesce into few sectors.  Small volumes split each tile's
-// pairs over up to 8 CTAs, whose partial volumes are added in pair order.  All pairs are used (the reference skips the last P mod
-// blockDim) and every voxel is visited for any N.
+// Layout: one CTA = 64 threads = a 4 x 4 x 16 voxel tile (z fastest, x slowest), the four
+// voxels of an x line per thread as two packed FP32x2 lane pairs (4 x 8 x 8: the same time at
+// 64^3, 24% more at 42 x 11 x 93).  Pair records are staged 64 at a time in shared memory,
+// coordinates doubled for the packed arithmetic, and read as warp-uniform broadcasts; a
+// warp's 128 voxels gather from one H row at neighbouring bins, so the global gathers
+// coalesce into few sectors.  Small volumes split each tile's pairs over up to 16 CTAs, whose
+// partial volumes are added in pair order.  All pairs are used (the reference skips the last
+// P mod blockDim) and every voxel is visited for any N.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,9 +44,9 @@
 namespace bpgb {
 namespace {
 
-constexpr int kTX = 4, kTY = 8, kTZ = 8;
+constexpr int kTX = 4, kTY = 4, kTZ = 16;
 constexpr int kThreads = kTY * kTZ;  // each thread owns the kTX voxels of an x line
-constexpr uint32_t kMaxSplits = 8;
+constexpr uint32_t kMaxSplits = 16;
 constexpr int kGroup = 64;           // pairs staged and marked together: two mask words
 
 struct ExactArgs {
@@ -371,10 +372,11 @@ uint32_t exact_splits(const Volume &vol, uint64_t P, int sm_count) {
     const uint64_t tiles = (uint64_t)((vol.n[0] + kTX - 1) / kTX) * ((vol.n[1] + kTY - 1) / kTY) *
                            ((vol.n[2] + kTZ - 1) / kTZ);
     // 16 CTAs (of 64 threads and 64 registers) fill an SM, and the gathers' latency wants them
-    // all: split until there are two rounds of them (1,024 tiles x 4,096 pairs: 1 split 1.24
-    // ms, 3 1.08, 5 0.974, 7 0.969), as long as a split keeps two groups of pairs.
+    // all and even last rounds: split until there are four rounds of them, as long as a split
+    // keeps two groups of pairs.  1,024 tiles x 4,096 pairs: 1 split 1.24 ms, 3 1.08, 5 0.970, 10
+    // 0.946; 42 x 11 x 93 voxels x 8,836 pairs: 8 splits 0.571 ms, 16 0.538.
     uint32_t s = 1;
-    while (tiles && s < kMaxSplits && s * tiles < 32ull * sm_count && P >= 2ull * (s + 1) * kGroup) s++;
+    while (tiles && s < kMaxSplits && s * tiles < 64ull * sm_count && P >= 2ull * (s + 1) * kGroup) s++;
     return s;
 }
 

@@ -66,7 +66,7 @@ struct ExactFilter {
 };
 ExactFilter exact_filter(const bpgb_pair *pairs, uint64_t P, const Volume &vol,
                          const BinParams &bp);
-// CTAs that share a voxel tile's pairs (1..8); above 1 d_partial holds that many volumes.
+// CTAs that share a voxel tile's pairs (1..16); above 1 d_partial holds that many volumes.
 uint32_t exact_splits(const Volume &vol, uint64_t P, int sm_count);
 int launch_exact(const void *d_H, bool is_complex, uint64_t pitch, const bpgb_pair *d_pairs,
                  uint64_t P, const Volume &vol, const BinParams &bp, const ExactFilter &filter,

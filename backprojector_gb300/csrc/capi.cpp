@@ -521,11 +521,11 @@ int bpgb_plan_get_info(bpgb_plan plan, bpgb_plan_info *info) {
     info->num_lasers = plan->fz.L;
     info->num_spads = plan->fz.S;
     info->tile[0] = 4;
-    info->tile[1] = 8;
-    info->tile[2] = 8;
+    info->tile[1] = 4;
+    info->tile[2] = 16;
     info->pair_splits = plan->splits;
-    info->grid = plan->splits * (uint32_t)(((plan->vol.n[0] + 3) / 4) * ((plan->vol.n[1] + 7) / 8) *
-                            ((plan->vol.n[2] + 7) / 8));
+    info->grid = plan->splits * (uint32_t)(((plan->vol.n[0] + 3) / 4) * ((plan->vol.n[1] + 3) / 4) *
+                            ((plan->vol.n[2] + 15) / 16));
     info->threads = 64;
     info->scratch_bytes = plan->P * sizeof(bpgb_pair) +
                           (plan->splits > 1 ? plan->splits * plan->vol.count() *
