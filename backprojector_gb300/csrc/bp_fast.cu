@@ -1928,17 +1928,23 @@ int fast_args(FastArgs &a, const FastConfig &cfg, const Volume &vol, const doubl
 }
 
 // Pair splits of a launch of `groups` CTAs per split over `items` work items each: the count,
-// up to six rounds of resident CTAs, whose busiest SM finishes first.  An SM takes n CTAs,
+// up to six rounds of resident CTAs (or eighteen, of at most eight splits: under 134 MB of
+// real partial sums), whose busiest SM finishes first.  An SM takes n CTAs,
 // `occ` at a time; a last round of r < occ CTAs, with fewer warps to hide latency, lasts like
 // r + 0.3 (occ - r) of them in a full round; a CTA's start-up costs about a quarter of an
 // item.  Those two constants were fitted to sixteen captures (8 to 720 tiles, every scan and
 // row type) timed at every split count: the rule's choice is 1.0% from the best on average
 // (at most 10%), where filling two rounds regardless of the remainder was 10% (32%): 64^3
 // voxels, 4,096 pairs, 8 -> 7 splits 322 -> 318 us; 34 x 62 x 14 voxels 39 -> 19 splits 36 ->
-// 27 us; lasers x SPADs at 32^3 38 -> 19 splits 453 -> 451 us.
+// 27 us; lasers x SPADs at 32^3 38 -> 19 splits 453 -> 451 us.  Past six rounds a large volume's
+// last round is still worth levelling (no size of 80^3 to 192^3, real or complex, over 1.2% from
+// its best count; up to 8% with six rounds): 4,096 pairs at 128^3 3 -> 4 splits 2.252 -> 2.175 ms,
+// at 144^3 2 -> 5 3.212 -> 3.081, 16,384 complex64 pairs at 96^3 2 -> 7 9.89 -> 9.34, at 128^3
+// 3 -> 4 19.26 -> 18.90.
 uint64_t auto_splits(uint64_t groups, uint64_t items, uint32_t sms, int occ) {
-    const uint64_t rounds = (6ull * sms * occ + groups - 1) / groups;
-    const uint64_t most = std::min<uint64_t>(items, std::max<uint64_t>(1, rounds));
+    const uint64_t six = (6ull * sms * occ + groups - 1) / groups;
+    const uint64_t eighteen = (18ull * sms * occ + groups - 1) / groups;
+    const uint64_t most = std::min(items, std::max(six, std::min<uint64_t>(eighteen, 8)));
     uint64_t best = 1;
     double best_cost = INFINITY;
     for (uint64_t s = 1; s <= most; s++) {
@@ -2125,11 +2131,20 @@ int fast_plan_build(FastPlan **out, const bpgb_pair *d_pairs, uint64_t P,
 
     // partial sums: [split][voxel] for full launches, [slot][split][tile voxel] for
     // tile-list launches (tiles x tile voxels >= voxels)
-    const size_t part_bytes =
+    size_t part_bytes =
         splits > 1 ? (size_t)splits * ntiles * a.tdim[0] * a.tdim[1] * a.tdim[2] *
                          (dt == BPGB_DTYPE_C64 || dt == BPGB_DTYPE_C32 ? 8 : 4)
                    : 0;
     if (part_bytes) e = cudaMalloc(&fp->d_partial, part_bytes);
+    if (e == cudaErrorMemoryAllocation && opt.pair_splits == 0) {
+        // the rule's own splits are for speed alone: without room for them, one
+        cudaGetLastError();
+        e = cudaSuccess;
+        part_bytes = 0;
+        a.splits = 1;
+        fp->grid = (uint32_t)ngroups;
+        fp->a = a;
+    }
     if (e != cudaSuccess) {
         fast_plan_free(fp);
         return e == cudaErrorMemoryAllocation ? set_error(BPGB_ERR_OUT_OF_MEMORY, "fast plan scratch")
