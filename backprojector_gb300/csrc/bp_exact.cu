@@ -21,7 +21,7 @@
 // marked pair per lane at a time, so that a warp spends one evaluation on the marks of all
 // its lanes.  E = 0.5 (scales where the bound does not hold) marks every update.
 //
-// Bound: issue (24 instructions per update, the marked ones' evaluations included) and the
+// Bound: issue (24 to 28 instructions per update, the marked ones' evaluations included) and the
 // latency of the L1 gathers.  Measured on 64 x 64 pairs that do not factor, T = 2048, 64^3
 // voxels: 3.60 ms before, 0.95 ms with the filter.
 //
