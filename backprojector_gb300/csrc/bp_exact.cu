@@ -255,7 +255,6 @@ template <typename HT>
 __global__ void exact_reduce_kernel(const HT *__restrict__ partial, HT *__restrict__ out,
                                     uint64_t nvox, uint32_t splits) {
     wait_previous();
-    allow_next();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= nvox) return;
     HT v[kMaxSplits];

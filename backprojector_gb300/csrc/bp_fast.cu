@@ -1393,7 +1393,6 @@ __global__ void __launch_bounds__(kReduceX *kReduceY)
     reduce_splits_kernel(const float *__restrict__ partial, float *__restrict__ out, uint64_t n,
                          uint32_t splits, float scale, int vec, int rows) {
     wait_previous();
-    allow_next();
     const uint64_t quads = (n + 3) / 4;
     const bool vp = vec && n % 4 == 0;  // every split's block is 16-byte aligned
     if (KAHAN || !rows) {

@@ -65,7 +65,6 @@ __global__ void __launch_bounds__(kMaxThreads)
                         uint32_t out_pitch, uint32_t nseg, int vec) {
     extern __shared__ __align__(16) float sm[];
     wait_previous();
-    allow_next();
     const int groups = blockDim.x + (min(K, kTapBlock) + kPer - 1) / kPer + 2;
     float4 *tp4 = reinterpret_cast<float4 *>(sm + (size_t)groups * kGroupWords);
     float2 *tp = reinterpret_cast<float2 *>(tp4);

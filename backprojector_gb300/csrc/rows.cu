@@ -41,7 +41,6 @@ template <bool VEC>
 __global__ void __launch_bounds__(256)
     absmax_kernel(const float *__restrict__ in, const Rows g, unsigned int *__restrict__ out) {
     wait_previous();
-    allow_next();
     unsigned int m = 0;
     auto take = [&](float v) { m = max(m, __float_as_uint(v) & 0x7fffffffu); };
     for (uint64_t q = blockIdx.x; q < g.rows * g.pieces; q += gridDim.x) {
@@ -89,7 +88,6 @@ __global__ void __launch_bounds__(256)
     to_half_kernel(const float *__restrict__ in, const Rows g, uint64_t T, float scale,
                    const float *__restrict__ d_absmax, float target, HT *__restrict__ out) {
     wait_previous();
-    allow_next();
     const float inv_scale = 1.0f / scale_of(scale, d_absmax, target);
     const uint64_t count = g.rows * g.pieces;
     for (uint64_t b = blockIdx.x; b < count; b += gridDim.x) {
@@ -135,7 +133,6 @@ __global__ void __launch_bounds__(256)
     scale_kernel(float *__restrict__ v, uint64_t n, float scale,
                  const float *__restrict__ d_absmax, float target) {
     wait_previous();
-    allow_next();
     const float f = scale_of(scale, d_absmax, target);
     const uint64_t step = (uint64_t)gridDim.x * 256, at = blockIdx.x * 256ull + threadIdx.x;
     uint64_t i = at;
