@@ -312,15 +312,23 @@ ExactArgs make_args(uint64_t pitch, uint64_t P, const Volume &vol, const BinPara
 
 ExactFilter exact_filter(const bpgb_pair *pairs, uint64_t P, const Volume &vol,
                          const BinParams &bp) {
-    // The largest legs, path and coordinate over the plan's pairs and voxels, in FP64.
+    // The largest legs, path and coordinate over the plan's pairs and voxels, in FP64.  The box
+    // holds the positions as the kernels round them: far from the origin they leave the box of
+    // the exact corners by up to 4 u (three FMAs and the index's conversion) of the largest sum
+    // on the way, which the relative error of the legs below does not cover.
     double lo[3], hi[3], size = 0.0, legs = 0.0, reach = 0.0, wall = 0.0, least = INFINITY;
     double near = INFINITY, far = -INFINITY;
     for (int k = 0; k < 3; k++) {
         lo[k] = hi[k] = vol.zero[k];
+        double sum = std::fabs((double)vol.zero[k]);
         for (int a = 0; a < 3; a++) {
             const double e = (double)vol.inc[3 * a + k] * (vol.n[a] ? vol.n[a] - 1 : 0);
             (e < 0.0 ? lo[k] : hi[k]) += e;
+            sum += std::fabs(e);
         }
+        const double rounding = 1.01 * std::ldexp(4.0, -24) * sum;
+        lo[k] -= rounding;
+        hi[k] += rounding;
         size = std::max({size, std::fabs(lo[k]), std::fabs(hi[k])});
     }
     auto nearest = [&](const float *p) {
