@@ -641,14 +641,18 @@ int bpgb_backproject_host(const void *transient_chunk, uint64_t transient_size, 
     thread_local DeviceBuffer dH, dV;
     st = dH.reserve(std::max<size_t>(16, num_pairs * (size_t)pitch * esz));
     if (!st) st = dV.reserve(std::max<size_t>(16, nvox * out_esz));
-    auto upload = [&](uint64_t r0, uint64_t r1, cudaStream_t s) {  // rows [r0, r1)
+    // Rows [r0, r1); on a stream of the call's own, or in the legacy default stream's order.
+    auto upload = [&](uint64_t r0, uint64_t r1, cudaStream_t s) {
         if (r1 <= r0) return cudaSuccess;
         char *dst = (char *)dH.ptr + r0 * pitch * esz;
         const char *src = (const char *)transient_chunk + r0 * T * esz;
-        return pitch == T ? cudaMemcpyAsync(dst, src, (r1 - r0) * (size_t)T * esz,
-                                            cudaMemcpyHostToDevice, s)
-                          : cudaMemcpy2DAsync(dst, pitch * esz, src, (size_t)T * esz, (size_t)T * esz,
-                                              r1 - r0, cudaMemcpyHostToDevice, s);
+        const size_t row = (size_t)T * esz, n = r1 - r0;
+        if (s)
+            return pitch == T ? cudaMemcpyAsync(dst, src, n * row, cudaMemcpyHostToDevice, s)
+                              : cudaMemcpy2DAsync(dst, pitch * esz, src, row, row, n,
+                                                  cudaMemcpyHostToDevice, s);
+        return pitch == T ? cudaMemcpy(dst, src, n * row, cudaMemcpyHostToDevice)
+                          : cudaMemcpy2D(dst, pitch * esz, src, row, row, n, cudaMemcpyHostToDevice);
     };
     // A large capture is uploaded in parts, the pair splits of each part running while the
     // next one is copied (4,096 x 2,048 FP32 rows into 64^3 voxels: 588 -> 512 us).
@@ -657,7 +661,10 @@ int bpgb_backproject_host(const void *transient_chunk, uint64_t transient_size, 
                                : 1;
     thread_local HostStreams hs;
     if (!st && parts > 1 && hs.ready()) {
-        cudaError_t e = cudaSuccess;
+        // The call's streams don't order themselves after the legacy default stream, as a
+        // synchronous copy does: work queued there may still be writing the rows.
+        cudaError_t e = cudaEventRecord(hs.event, cudaStreamLegacy);
+        if (e == cudaSuccess) e = cudaEventSynchronize(hs.event);
         uint64_t row = 0;
         for (uint32_t k = 0; k < parts && e == cudaSuccess && !st; k++) {
             const uint64_t end = fast_plan_part_rows(plan->fast, k, parts);

@@ -136,7 +136,8 @@ uint64_t bpgb_launch_count(void);
 /* ---- drop-in host-buffer calls ------------------------------------------
  * Same arguments and meaning as the reference: caller-owned HOST buffers,
  * transient_size = P * T elements, the voxel volume [Nx, Ny, Nz] (x slowest) is
- * OVERWRITTEN, the call is synchronous on the current device.  Unlike the reference,
+ * OVERWRITTEN, the call is synchronous on the current device and, as a synchronous copy is,
+ * ordered after the work queued in the legacy default stream.  Unlike the reference,
  * every pair is used (it skips the last P mod blockDim pairs) and every voxel is
  * visited exactly once for any N (its voxel cursor wraps and recomputes some voxels
  * when N is not a multiple of 16, backproject_cuda.cu:65-80).
