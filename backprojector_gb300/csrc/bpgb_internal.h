@@ -169,13 +169,4 @@ int launch_pairs_fp64(const float *d_laser_grid, uint32_t lx, uint32_t ly,
                       const double *laser_pos, const double *camera_pos, int confocal,
                       bpgb_pair *d_out, cudaStream_t stream);
 
-// ---- device memory cache for the host-buffer entry points ----------------------
-// Grow-only per-thread buffers reused across calls (avoids cudaMalloc per call).
-struct DeviceBuffer {
-    void *ptr = nullptr;
-    size_t bytes = 0;
-    int reserve(size_t need);
-    ~DeviceBuffer();
-};
-
 }  // namespace bpgb

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "bpgb_internal.h"
+#include "host_cache.h"
 
 using namespace bpgb;
 
