@@ -250,6 +250,46 @@ __global__ void __launch_bounds__(kThreads)
             out[((uint64_t)(x + w) * a.n[1] + y) * a.n[2] + z] = acc[w];
 }
 
+// Plans whose cheap quotient is not trusted: the reference's expression for every update, one
+// voxel of a 4 x 8 x 8 tile per thread, pairs staged 256 at a time.  Bound by issue (about 100
+// instructions per update).  It doesn't call allow_next: 6.7 CTAs per SM of 64^3 voxels are
+// placed unevenly around a pass's own (80 pairs, a pass among others: 77.6 us with early starts,
+// 68.8 without; 63.7 with the split's first pair and row added to the pointers once).
+constexpr int kDirectX = 4, kDirectY = 8, kDirectZ = 8;
+constexpr int kDirectThreads = kDirectX * kDirectY * kDirectZ;
+template <typename HT>
+__global__ void __launch_bounds__(kDirectThreads)
+    bp_exact_direct_kernel(const HT *__restrict__ H, const bpgb_pair *__restrict__ pairs,
+                           HT *__restrict__ out, const ExactArgs a) {
+    wait_previous();
+    __shared__ bpgb_pair sp[kDirectThreads];
+    uint32_t t = blockIdx.x / a.splits;
+    const uint32_t z = t % a.tiles[2] * kDirectZ + threadIdx.x % kDirectZ;
+    t /= a.tiles[2];
+    const uint32_t x = t % a.tiles[0] * kDirectX + threadIdx.x / (kDirectZ * kDirectY);
+    const uint32_t y = t / a.tiles[0] * kDirectY + threadIdx.x / kDirectZ % kDirectY;
+    float v[3];
+    voxel_position(a, x, y, z, v);
+    HT acc = zero_h<HT>();
+    const int last = (int)a.T - 1;
+    const uint32_t split = blockIdx.x % a.splits;
+    const uint64_t p0 = a.P * split / a.splits, P = a.P * (split + 1) / a.splits - p0;
+    H += p0 * a.pitch;
+    pairs += p0;
+    for (uint64_t base = 0; base < P; base += kDirectThreads) {
+        __syncthreads();
+        if (base + threadIdx.x < P) sp[threadIdx.x] = pairs[base + threadIdx.x];
+        __syncthreads();
+        const uint32_t n = (uint32_t)min((uint64_t)kDirectThreads, P - base);
+        for (uint32_t j = 0; j < n; j++) {
+            const int b = exact_bin(sp[j], v, a.t0, a.dT);
+            if (b >= 0 && b <= last) add_to(acc, load_h(H, (base + j) * a.pitch + (uint64_t)b));
+        }
+    }
+    if (x < a.n[0] && y < a.n[1] && z < a.n[2])
+        out[split * a.nvox + ((uint64_t)x * a.n[1] + y) * a.n[2] + z] = acc;
+}
+
 // out = the splits' partial sums, added in pair order.
 template <typename HT>
 __global__ void exact_reduce_kernel(const HT *__restrict__ partial, HT *__restrict__ out,
@@ -295,9 +335,6 @@ ExactArgs make_args(uint64_t pitch, uint64_t P, const Volume &vol, const BinPara
         a.zero[k] = vol.zero[k];
     }
     for (int k = 0; k < 9; k++) a.inc[k] = vol.inc[k];
-    a.tiles[0] = (vol.n[0] + kTX - 1) / kTX;
-    a.tiles[1] = (vol.n[1] + kTY - 1) / kTY;
-    a.tiles[2] = (vol.n[2] + kTZ - 1) / kTZ;
     a.t0 = bp.t0;
     a.dT = bp.dT;
     a.T = bp.T;
@@ -375,38 +412,68 @@ ExactFilter exact_filter(const bpgb_pair *pairs, uint64_t P, const Volume &vol,
     return f;
 }
 
-uint32_t exact_splits(const Volume &vol, uint64_t P, int sm_count) {
-    const uint64_t tiles = (uint64_t)((vol.n[0] + kTX - 1) / kTX) * ((vol.n[1] + kTY - 1) / kTY) *
-                           ((vol.n[2] + kTZ - 1) / kTZ);
-    // 16 CTAs (of 64 threads and 64 registers) fill an SM, and the gathers' latency wants them
-    // all and even last rounds: split until there are four rounds of them, as long as a split
-    // keeps two groups of pairs.  1,024 tiles x 4,096 pairs: 1 split 1.24 ms, 3 1.08, 5 0.970, 10
-    // 0.946; 42 x 11 x 93 voxels x 8,836 pairs: 8 splits 0.571 ms, 16 0.538.
-    uint32_t s = 1;
-    while (tiles && s < kMaxSplits && s * tiles < 64ull * sm_count && P >= 2ull * (s + 1) * kGroup) s++;
-    return s;
+ExactShape exact_shape(const Volume &vol, uint64_t P, const ExactFilter &filter, int sm_count) {
+    auto shape = [&](bool direct, uint32_t tx, uint32_t ty, uint32_t tz, uint32_t threads,
+                     uint64_t ctas, uint64_t pairs) {
+        ExactShape e;
+        const uint32_t t[3] = {tx, ty, tz};
+        e.direct = direct;
+        e.threads = threads;
+        e.ctas = 1;
+        for (int k = 0; k < 3; k++) {
+            e.tile[k] = t[k];
+            e.tiles[k] = (vol.n[k] + t[k] - 1) / t[k];
+            e.ctas *= e.tiles[k];
+        }
+        // up to `ctas` per SM, as long as a split keeps `pairs` of them
+        const uint64_t tiles = e.ctas;
+        while (tiles && e.splits < kMaxSplits && e.splits * tiles < ctas * sm_count &&
+               P >= pairs * (e.splits + 1))
+            e.splits++;
+        e.ctas = tiles * e.splits;
+        return e;
+    };
+    // The gathers' latency wants every SM's slots (13 or 14 CTAs of 64 threads) full and an even
+    // last round, and a split two groups of pairs.  1,024 tiles x 4,096 pairs: 1 split 1.24 ms,
+    // 3 1.08, 5 0.970, 10 0.946; 42 x 11 x 93 voxels x 8,836 pairs: 8 splits 0.571 ms, 16 0.538.
+    const ExactShape filtered = shape(false, kTX, kTY, kTZ, kThreads, 64, 2 * kGroup);
+    // Direct: an even last round of 8 CTAs per SM (64^3 voxels x 1,024 pairs: 1 split 782 us, 2 766,
+    // 4 710).
+    const ExactShape direct = shape(true, kDirectX, kDirectY, kDirectZ, kDirectThreads, 24, 64);
+    // Quotients that are not trusted would all be computed and then marked (64^3 voxels x 1,024
+    // pairs: 1,680 us against 710; 2 x 16 x 3 voxels x 170 pairs: 211 us against 23).  Above a mark
+    // per 50 updates a launch of few CTAs waits for the marks, too (69 x 7 x 11 voxels x 80 pairs in
+    // bins of 0.3 mm: 24.9 us against 20.0), where one that fills the GPU does not (64^3 voxels x
+    // 80 pairs: 39.7 us against 63.7).
+    if (!(filter.error < 0.5f) || filtered.ctas > 0x7fffffffull ||
+        (filter.error > 0.01f && filtered.ctas < 2ull * sm_count))
+        return direct;
+    return filtered;
 }
 
 int launch_exact(const void *d_H, bool is_complex, uint64_t pitch, const bpgb_pair *d_pairs,
                  uint64_t P, const Volume &vol, const BinParams &bp, const ExactFilter &filter,
-                 uint32_t splits, void *d_partial, void *d_out, cudaStream_t stream) {
+                 const ExactShape &shape, void *d_partial, void *d_out, cudaStream_t stream) {
     ExactArgs a = make_args(pitch, P, vol, bp);
+    const uint32_t splits = shape.splits;
+    for (int k = 0; k < 3; k++) a.tiles[k] = shape.tiles[k];
     a.inv = 1.0f / bp.dT;
     a.invd = 1.0 / (double)bp.dT;
     a.thr = 0.5f - filter.error;
     a.half = 0.5f * (float)(bp.T - 1);
     a.splits = splits;
-    const uint64_t tiles = (uint64_t)a.tiles[0] * a.tiles[1] * a.tiles[2];
-    if (tiles == 0) return BPGB_OK;
-    if (tiles * splits > 0x7fffffffull)
+    if (shape.ctas == 0) return BPGB_OK;
+    if (shape.ctas > 0x7fffffffull)
         return set_error(BPGB_ERR_UNSUPPORTED, "volume too large for the exact kernel grid");
     void *target = splits > 1 ? d_partial : d_out;
     void *args[] = {(void *)&d_H, (void *)&d_pairs, (void *)&target, (void *)&a};
-    void *kern = is_complex ? (filter.inside ? (void *)bp_exact_kernel<float2, true>
-                                             : (void *)bp_exact_kernel<float2, false>)
-                            : (filter.inside ? (void *)bp_exact_kernel<float, true>
-                                             : (void *)bp_exact_kernel<float, false>);
-    BPGB_CUDA_TRY(launch_after(kern, (unsigned)(tiles * splits), kThreads, args, 0, stream));
+    void *kern = shape.direct ? (is_complex ? (void *)bp_exact_direct_kernel<float2>
+                                            : (void *)bp_exact_direct_kernel<float>)
+                 : is_complex ? (filter.inside ? (void *)bp_exact_kernel<float2, true>
+                                               : (void *)bp_exact_kernel<float2, false>)
+                              : (filter.inside ? (void *)bp_exact_kernel<float, true>
+                                               : (void *)bp_exact_kernel<float, false>);
+    BPGB_CUDA_TRY(launch_after(kern, (unsigned)shape.ctas, shape.threads, args, 0, stream));
     count_launches(1);
     if (splits > 1) {
         const unsigned blocks = (unsigned)((a.nvox + 255) / 256);

@@ -57,7 +57,6 @@ struct BinParams {
 };
 
 // ---- exact kernels (bp_exact.cu) ----------------------------------------------
-// H rows of `pitch` elements, float or interleaved complex64 (is_complex).
 // Bound (bins) on the distance between the kernel's cheap quotient and the reference's over
 // a plan's pairs and voxels; 0.5 where none holds (every update is then evaluated in full).
 struct ExactFilter {
@@ -66,11 +65,19 @@ struct ExactFilter {
 };
 ExactFilter exact_filter(const bpgb_pair *pairs, uint64_t P, const Volume &vol,
                          const BinParams &bp);
-// CTAs that share a voxel tile's pairs (1..16); above 1 d_partial holds that many volumes.
-uint32_t exact_splits(const Volume &vol, uint64_t P, int sm_count);
+// A plan's kernel and launch shape.
+struct ExactShape {
+    bool direct = false;  // the reference's expression for every update, no cheap quotient
+    uint32_t tile[3] = {1, 1, 1}, tiles[3] = {0, 0, 0}, threads = 0;
+    uint32_t splits = 1;  // CTAs that share a tile's pairs (1..16); above 1 d_partial holds that
+                          // many volumes
+    uint64_t ctas = 0;    // tiles x splits
+};
+ExactShape exact_shape(const Volume &vol, uint64_t P, const ExactFilter &filter, int sm_count);
+// H rows of `pitch` elements, float or interleaved complex64 (is_complex).
 int launch_exact(const void *d_H, bool is_complex, uint64_t pitch, const bpgb_pair *d_pairs,
                  uint64_t P, const Volume &vol, const BinParams &bp, const ExactFilter &filter,
-                 uint32_t splits, void *d_partial, void *d_out, cudaStream_t stream);
+                 const ExactShape &shape, void *d_partial, void *d_out, cudaStream_t stream);
 int launch_exact_bins(const bpgb_pair *d_pairs, uint64_t P, const Volume &vol,
                       const BinParams &bp, const int64_t *d_ids, int64_t n, int32_t *d_bins,
                       cudaStream_t stream);

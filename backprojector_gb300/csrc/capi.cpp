@@ -230,9 +230,9 @@ struct bpgb_plan_s {
     Factorization fz{};
     bpgb_pair *d_pairs = nullptr;
     FastPlan *fast = nullptr;
-    ExactFilter filter{};  // EXACT
-    uint32_t splits = 1;         // EXACT: CTAs per voxel tile
-    void *d_partial = nullptr;   // EXACT: their partial volumes
+    ExactFilter filter{};       // EXACT, with the next two
+    ExactShape shape{};
+    void *d_partial = nullptr;  // the pair splits' partial volumes
     cudaStream_t last_stream = nullptr;
 };
 
@@ -359,13 +359,14 @@ int bpgb_plan_create(bpgb_plan *plan, const bpgb_pair *host_pairs, uint64_t num_
     p->algo = algo;
     if (algo == BPGB_ALGO_EXACT) {
         p->filter = exact_filter(host_pairs, num_pairs, p->vol, p->bp);
-        p->splits = exact_splits(p->vol, num_pairs, sms);
-        if (p->splits > 1) {
+        p->shape = exact_shape(p->vol, num_pairs, p->filter, sms);
+        if (p->shape.splits > 1) {
             const size_t esz = o.h_dtype == BPGB_DTYPE_C64 ? 8 : 4;
-            if (cudaMalloc(&p->d_partial, p->splits * p->vol.count() * esz) != cudaSuccess) {
+            if (cudaMalloc(&p->d_partial, p->shape.splits * p->vol.count() * esz) != cudaSuccess) {
                 cudaGetLastError();  // no room for partial volumes: one CTA per tile
                 p->d_partial = nullptr;
-                p->splits = 1;
+                p->shape.ctas /= p->shape.splits;
+                p->shape.splits = 1;
             }
         }
     }
@@ -388,7 +389,7 @@ int bpgb_plan_execute(bpgb_plan plan, const void *d_H, void *d_volume, void *str
     if (plan->algo == BPGB_ALGO_FAST) return fast_plan_execute(plan->fast, d_H, d_volume, s);
     const uint64_t pitch = plan->opt.h_pitch ? plan->opt.h_pitch : plan->bp.T;
     int st = launch_exact(d_H, cplx, pitch, plan->d_pairs, plan->P, plan->vol, plan->bp,
-                          plan->filter, plan->splits, plan->d_partial, d_volume, s);
+                          plan->filter, plan->shape, plan->d_partial, d_volume, s);
     if (st) return st;
     if (plan->opt.h_scale != 1.0f && plan->opt.h_scale != 0.0f)
         return set_error(BPGB_ERR_UNSUPPORTED, "h_scale applies to the FAST path only");
@@ -452,17 +453,15 @@ int bpgb_plan_get_info(bpgb_plan plan, bpgb_plan_info *info) {
     info->geometry = plan->fz.geom;
     info->num_lasers = plan->fz.L;
     info->num_spads = plan->fz.S;
-    info->tile[0] = 4;
-    info->tile[1] = 4;
-    info->tile[2] = 16;
-    info->pair_splits = plan->splits;
-    info->grid = plan->splits * (uint32_t)(((plan->vol.n[0] + 3) / 4) * ((plan->vol.n[1] + 3) / 4) *
-                            ((plan->vol.n[2] + 15) / 16));
-    info->threads = 64;
+    const ExactShape &e = plan->shape;
+    for (int k = 0; k < 3; k++) info->tile[k] = e.tile[k];
+    info->pair_splits = e.splits;
+    info->grid = (uint32_t)e.ctas;
+    info->threads = e.threads;
     info->scratch_bytes = plan->P * sizeof(bpgb_pair) +
-                          (plan->splits > 1 ? plan->splits * plan->vol.count() *
-                                                  (plan->opt.h_dtype == BPGB_DTYPE_C64 ? 8 : 4)
-                                            : 0);
+                          (e.splits > 1 ? e.splits * plan->vol.count() *
+                                              (plan->opt.h_dtype == BPGB_DTYPE_C64 ? 8 : 4)
+                                        : 0);
     return BPGB_OK;
 }
 
