@@ -13,26 +13,104 @@ namespace bpgb {
 namespace {
 
 // These passes move each byte once, so they are bound by HBM and need wide accesses in flight:
-// rows are cut into pieces of kPiece elements, one per CTA at a time and four or eight elements
+// rows are cut into pieces, one per CTA at a time and four or eight elements
 // per thread, and rows that follow one another without padding are taken as one long row.
 // 16,384 x 4,096 FP32 rows: absmax 137 -> 42 us, FP16 conversion 164 -> 54 us, scaling
 // a 256^3 volume 29 -> 15 us (one element and a 64-bit division per thread before).
-constexpr uint32_t kPiece = 1u << 14;
+constexpr uint32_t kMaxPiece = 1u << 14, kMinPiece = 1u << 10;
+constexpr uint32_t kSms = 152;
 
 struct Rows {
     uint64_t rows, T;   // T elements each
-    uint64_t pieces;    // of kPiece elements per row
+    uint64_t pieces;    // of `piece` elements per row
     uint64_t pitch;     // of the input
+    uint32_t piece;
 };
 
+// Few rows are cut finer, until every SM has two pieces (37 rows of 60,001 elements as FP16
+// 13.5 -> 4.1 us); more pieces cost long rows more (6.2 M elements' largest: 6.3 us, 6.7 with eight).
 Rows rows_of(uint64_t rows, uint64_t T, uint64_t pitch, bool flat) {
     if (flat) T *= rows, rows = 1, pitch = T;
-    return {rows, T, (T + kPiece - 1) / kPiece, pitch};
+    uint32_t piece = kMaxPiece;
+    while (piece > kMinPiece && rows * ((T + piece - 1) / piece) < 2 * kSms) piece /= 2;
+    return {rows, T, (T + piece - 1) / piece, pitch, piece};
 }
 
 unsigned blocks_for(const Rows &g) {
     const uint64_t n = g.rows * g.pieces;
-    return (unsigned)(n < 152 * 16 ? n : 152 * 16);
+    return (unsigned)(n < kSms * 16 ? n : kSms * 16);
+}
+
+// Padded rows too short to occupy a CTA each share one: `lanes` threads per row, up to four
+// elements each, and four rows of a thread in flight.  A CTA per row took 121 us for the
+// largest of 200,000 rows of 8 elements and 116 us for their conversion, against 12.3 and 8.2 us with
+// one element and a division per thread; 6.2 and 5.9 us now.
+constexpr uint32_t kShortRow = 512;
+constexpr uint32_t kRowsInFlight = 4;
+
+struct ShortRows {
+    uint64_t rows;
+    uint32_t T, pitch, lanes;  // a power of two
+
+    uint64_t units() const {  // of kRowsInFlight rows per thread
+        const uint64_t per = kRowsInFlight * (256 / lanes);
+        return (rows + per - 1) / per;
+    }
+};
+
+ShortRows short_rows(uint64_t rows, uint32_t T, uint32_t pitch, uint32_t width) {
+    ShortRows g{rows, T, pitch, 1};
+    while (g.lanes < 256 && g.lanes < width) g.lanes *= 2;
+    // fewer threads per row, down to a warp, where the rows still make eight CTAs per SM
+    while (g.lanes > 32 && 2 * g.lanes >= width) {
+        ShortRows h = g;
+        h.lanes /= 2;
+        if (h.units() < 8 * kSms) break;
+        g = h;
+    }
+    return g;
+}
+
+unsigned blocks_for(const ShortRows &g) {
+    const uint64_t n = g.units();
+    return (unsigned)(n < kSms * 16 ? n : kSms * 16);
+}
+
+__device__ __forceinline__ uint64_t short_row(const ShortRows &g, uint64_t unit, uint32_t k) {
+    return (unit * kRowsInFlight + k) * (256 / g.lanes) + threadIdx.x / g.lanes;
+}
+
+// The CTA's largest |value| as float bits into out[0] (NaN counts as +inf).
+__device__ __forceinline__ void block_max(unsigned int m, unsigned int *out) {
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ unsigned int warp_max[8];
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) m = max(m, warp_max[w]);
+        atomicMax(out, min(m, 0x7f800000u));
+    }
+}
+
+__global__ void __launch_bounds__(256)
+    absmax_short_kernel(const float *__restrict__ in, const ShortRows g, uint64_t units,
+                        unsigned int *__restrict__ out) {
+    wait_previous();
+    unsigned int m = 0;
+    for (uint64_t q = blockIdx.x; q < units; q += gridDim.x)
+#pragma unroll 2
+        for (uint32_t t = threadIdx.x & (g.lanes - 1); t < g.T; t += g.lanes) {
+            float v[kRowsInFlight];
+#pragma unroll
+            for (uint32_t k = 0; k < kRowsInFlight; k++) {
+                const uint64_t r = short_row(g, q, k);
+                v[k] = r < g.rows ? __ldg(in + r * g.pitch + t) : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kRowsInFlight; k++)
+                m = max(m, __float_as_uint(v[k]) & 0x7fffffffu);
+        }
+    block_max(m, out);
 }
 
 // out[0] = max |in| (float bits compare as unsigned for |x|; NaN counts as +inf).  VEC: rows
@@ -44,9 +122,9 @@ __global__ void __launch_bounds__(256)
     unsigned int m = 0;
     auto take = [&](float v) { m = max(m, __float_as_uint(v) & 0x7fffffffu); };
     for (uint64_t q = blockIdx.x; q < g.rows * g.pieces; q += gridDim.x) {
-        const uint64_t r = q / g.pieces, t0 = (q - r * g.pieces) * kPiece;
+        const uint64_t r = q / g.pieces, t0 = (q - r * g.pieces) * g.piece;
         const float *row = in + r * g.pitch + t0;
-        const uint32_t T = (uint32_t)min((uint64_t)kPiece, g.T - t0);
+        const uint32_t T = (uint32_t)min((uint64_t)g.piece, g.T - t0);
         uint32_t t = 0;
         if (VEC) {
             const float4 *row4 = reinterpret_cast<const float4 *>(row);
@@ -59,14 +137,7 @@ __global__ void __launch_bounds__(256)
         }
         for (t += threadIdx.x; t < T; t += 256) take(row[t]);
     }
-    m = __reduce_max_sync(0xffffffffu, m);
-    __shared__ unsigned int warp_max[8];
-    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; w++) m = max(m, warp_max[w]);
-        atomicMax(out, min(m, 0x7f800000u));
-    }
+    block_max(m, out);
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b, __half) {
@@ -91,10 +162,10 @@ __global__ void __launch_bounds__(256)
     const float inv_scale = 1.0f / scale_of(scale, d_absmax, target);
     const uint64_t count = g.rows * g.pieces;
     for (uint64_t b = blockIdx.x; b < count; b += gridDim.x) {
-        const uint64_t q = count - 1 - b, r = q / g.pieces, t0 = (q - r * g.pieces) * kPiece;
+        const uint64_t q = count - 1 - b, r = q / g.pieces, t0 = (q - r * g.pieces) * g.piece;
         const float *src = in + r * g.pitch + t0;
         HT *dst = out + r * g.T + t0;
-        const uint32_t n = (uint32_t)min((uint64_t)kPiece, g.T - t0);
+        const uint32_t n = (uint32_t)min((uint64_t)g.piece, g.T - t0);
         const uint32_t m = t0 < T ? (uint32_t)min((uint64_t)n, T - t0) : 0u;  // from the input
         uint32_t t = 0;
         if (VEC) {
@@ -111,8 +182,33 @@ __global__ void __launch_bounds__(256)
             }
             t = m / 8 * 8;
         }
-        for (t += threadIdx.x; t < n; t += 256) store_h(dst + t, t < m ? src[t] * inv_scale : 0.0f);
+#pragma unroll 4
+        for (t += threadIdx.x; t < n; t += 256) store_h(dst + t, t < m ? __ldg(src + t) * inv_scale : 0.0f);
     }
+}
+
+// The same for short padded rows.
+template <typename HT>
+__global__ void __launch_bounds__(256)
+    to_half_short_kernel(const float *__restrict__ in, const ShortRows g, uint64_t units,
+                         uint32_t out_pitch, float scale, const float *__restrict__ d_absmax,
+                         float target, HT *__restrict__ out) {
+    wait_previous();
+    const float inv_scale = 1.0f / scale_of(scale, d_absmax, target);
+    for (uint64_t q = blockIdx.x; q < units; q += gridDim.x)
+        for (uint32_t t = threadIdx.x & (g.lanes - 1); t < out_pitch; t += g.lanes) {
+            float v[kRowsInFlight];
+#pragma unroll
+            for (uint32_t k = 0; k < kRowsInFlight; k++) {
+                const uint64_t r = short_row(g, q, k);
+                v[k] = r < g.rows && t < g.T ? __ldg(in + r * g.pitch + t) * inv_scale : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kRowsInFlight; k++) {
+                const uint64_t r = short_row(g, q, k);
+                if (r < g.rows) store_h(out + r * out_pitch + t, v[k]);
+            }
+        }
 }
 
 // out[r][t] = in[r][from + t] for 0 <= from + t < T, else 0 (t < out_pitch).
@@ -167,6 +263,14 @@ int bpgb_rows_absmax(const float *d_H, uint64_t rows, uint32_t T, uint32_t pitch
     BPGB_CUDA_TRY(cudaMemsetAsync(d_max, 0, sizeof(float), s));
     const uint64_t n = rows * T;
     if (n == 0) return BPGB_OK;
+    if (rows > 1 && pitch != T && T <= kShortRow) {
+        const ShortRows g = short_rows(rows, T, pitch, T);
+        launch_after(absmax_short_kernel, blocks_for(g), 256, 0, s, d_H, g, g.units(),
+                     (unsigned int *)d_max);
+        count_launches(1);
+        BPGB_CUDA_TRY(cudaGetLastError());
+        return BPGB_OK;
+    }
     const Rows g = rows_of(rows, T, pitch, pitch == T);
     if (aligned16(d_H) && (g.rows == 1 || pitch % 4 == 0))
         launch_after(absmax_kernel<true>, blocks_for(g), 256, 0, s, d_H, g, (unsigned int *)d_max);
@@ -189,6 +293,18 @@ int bpgb_rows_to_half(const float *d_H, uint64_t rows, uint32_t T, uint32_t in_p
     if (n == 0) return BPGB_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const bool flat = in_pitch == T && out_pitch == T;
+    if (rows > 1 && !flat && out_pitch <= kShortRow) {
+        const ShortRows g = short_rows(rows, T, in_pitch, out_pitch);
+        auto run = [&](auto kernel, auto *out) {
+            launch_after(kernel, blocks_for(g), 256, 0, s, d_H, g, g.units(), out_pitch, scale, d_absmax,
+                         target, out);
+        };
+        dtype == BPGB_DTYPE_F16 ? run(to_half_short_kernel<__half>, (__half *)d_out)
+                                : run(to_half_short_kernel<__nv_bfloat16>, (__nv_bfloat16 *)d_out);
+        count_launches(1);
+        BPGB_CUDA_TRY(cudaGetLastError());
+        return BPGB_OK;
+    }
     const Rows g = rows_of(rows, out_pitch, in_pitch, flat);
     const bool vec = aligned16(d_H) && aligned16(d_out) &&
                      (g.rows == 1 || (in_pitch % 4 == 0 && out_pitch % 8 == 0));
