@@ -12,7 +12,8 @@
 // stages one row segment plus its halo in shared memory (zeros outside (0, T), which
 // reproduces the index test), groups of 8 values 48 bytes apart so that the lanes' 16-byte
 // loads hit distinct banks.  Measured on 16,384 rows of 4,096 bins and 503 taps: 4.79 ms
-// before, 3.94 ms now (3.4 ms at 128 FP32 results per SM and clock).  Packed FP32x2 sums
+// with strided outputs, 3.96 with a window of registers, 3.87 with one for the last K mod 8 taps
+// too (3.4 ms at 128 FP32 results per SM and clock; 71 taps 0.768 -> 0.627 ms).  Packed FP32x2 sums
 // measured 4.12 ms; packed products are fused with packed sums whatever their rounding
 // modifiers, which changes bits.
 #include <cuda_runtime.h>
@@ -59,6 +60,8 @@ __device__ __forceinline__ void mul_add(float2 &acc, float x, float2 c) {
     acc.y = __fadd_rn(acc.y, __fmul_rn(x, c.y));
 }
 
+// REST: K is not a multiple of kPer.
+template <bool REST>
 __global__ void __launch_bounds__(kMaxThreads)
     phasor_pulse_kernel(const float *__restrict__ H, uint32_t T, uint32_t in_pitch,
                         const float2 *__restrict__ taps, int K, float2 *__restrict__ out,
@@ -112,13 +115,16 @@ __global__ void __launch_bounds__(kMaxThreads)
 #pragma unroll
             for (int j = 0; j < kPer; j++) x0[j] = x1[j];
         }
-        for (int k = full * kPer; k < kt; k++) {  // the last K mod 8 taps
-            const float2 c = tp[k];
+        if (!REST) continue;
+        const int rest = kt - full * kPer;  // the last K mod 8 taps
+        if (rest) load_group(threadIdx.x + full + 1, x1);
 #pragma unroll
-            for (int j = 0; j < kPer; j++) {
-                const int i = threadIdx.x * kPer + k + j;
-                mul_add(acc[j], sm[(i / kPer) * kGroupWords + i % kPer], c);
-            }
+        for (int u = 0; u < kPer - 1; u++) {
+            if (u >= rest) break;
+            const float2 c = tp[full * kPer + u];
+#pragma unroll
+            for (int j = 0; j < kPer; j++)
+                mul_add(acc[j], u + j < kPer ? x0[u + j] : x1[u + j - kPer], c);
         }
     }
     const int64_t t = t_begin + threadIdx.x * kPer;
@@ -132,6 +138,44 @@ __global__ void __launch_bounds__(kMaxThreads)
 #pragma unroll
         for (int j = 0; j < kPer; j++)
             if (t + j < (int64_t)T) o[j] = acc[j];
+    }
+}
+
+// Few taps (K < kFewTaps): bound by the rows' and the field's bytes, so outputs strided by the
+// block, whose loads and stores are contiguous across a warp and need little preparation.
+// 16,384 x 4,096, this kernel against the one above: 3 taps 124 / 192 us, 15 211 / 240, 28 321 / 331, 31
+// 354 / 348.  The block's size is a template argument (8 taps 155 us, 181 without).
+constexpr int kFewTaps = 31;
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    phasor_few_taps_kernel(const float *__restrict__ H, uint32_t T, uint32_t in_pitch,
+                           const float2 *__restrict__ taps, int K, float2 *__restrict__ out,
+                           uint32_t out_pitch, uint32_t nseg) {
+    __shared__ float seg[THREADS * kPer + kFewTaps];
+    __shared__ float2 tp[kFewTaps];
+    wait_previous();
+    const uint64_t r = blockIdx.x / nseg;
+    const int64_t t_begin = (int64_t)(blockIdx.x % nseg) * THREADS * kPer;
+    const float *row = H + r * in_pitch;
+    for (int i = threadIdx.x; i < THREADS * kPer + K; i += THREADS) {
+        const int64_t ri = t_begin - K / 2 + i;
+        seg[i] = (ri > 0 && ri < (int64_t)T) ? row[ri] : 0.0f;
+    }
+    for (int k = threadIdx.x; k < K; k += THREADS) tp[k] = taps[k];
+    __syncthreads();
+    float2 acc[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; j++) acc[j] = make_float2(0.0f, 0.0f);
+    for (int k = 0; k < K; k++) {
+        const float2 c = tp[k];
+#pragma unroll
+        for (int j = 0; j < kPer; j++) mul_add(acc[j], seg[threadIdx.x + j * THREADS + k], c);
+    }
+    float2 *orow = out + r * out_pitch;
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        const int64_t t = t_begin + threadIdx.x + j * THREADS;
+        if (t < (int64_t)T) orow[t] = acc[j];
     }
 }
 
@@ -179,15 +223,29 @@ int launch_phasor_pulse(const float *d_H, uint64_t rows, uint32_t T, uint32_t in
         return BPGB_OK;
     }
     const PulseShape p = pulse_shape(T, K);
-    if ((size_t)(((kSeg + K + 1) & ~1) + 2 * K) * sizeof(float) > 200 * 1024) return set_error(BPGB_ERR_UNSUPPORTED, "phasor pulse too long");
+    // the limit of callers' pulses (about 16,700 taps), not of these kernels
+    if ((size_t)(((kSeg + K + 1) & ~1) + 2 * K) * sizeof(float) > 200 * 1024)
+        return set_error(BPGB_ERR_UNSUPPORTED, "phasor pulse too long");
     const uint64_t blocks = rows * p.nseg;
     if (blocks >= (1ull << 31)) return set_error(BPGB_ERR_UNSUPPORTED, "too many rows for one launch");
     const float2 *d_taps = nullptr;
     if (int st = device_taps(h_taps, K, &d_taps)) return st;
-    if (int rs = reserve_dynamic_smem((const void *)phasor_pulse_kernel, p.smem)) return rs;
+    if (K < kFewTaps) {
+        const auto few = p.threads == 32  ? phasor_few_taps_kernel<32>
+                         : p.threads == 64 ? phasor_few_taps_kernel<64>
+                         : p.threads == 96 ? phasor_few_taps_kernel<96>
+                                           : phasor_few_taps_kernel<128>;
+        launch_after(few, (unsigned)blocks, p.threads, 0, stream, d_H, T, in_pitch,
+                     d_taps, K, reinterpret_cast<float2 *>(d_out), out_pitch, p.nseg);
+        count_launches(1);
+        BPGB_CUDA_TRY(cudaGetLastError());
+        return BPGB_OK;
+    }
+    const auto kernel = K % kPer ? phasor_pulse_kernel<true> : phasor_pulse_kernel<false>;
+    if (int rs = reserve_dynamic_smem((const void *)kernel, p.smem)) return rs;
     // 16-byte stores where every row's outputs are 16-byte aligned
     const int vec = ((uintptr_t)d_out % 16 == 0 && out_pitch % 2 == 0) ? 1 : 0;
-    launch_after(phasor_pulse_kernel, (unsigned)blocks, p.threads, p.smem, stream, d_H, T, in_pitch,
+    launch_after(kernel, (unsigned)blocks, p.threads, p.smem, stream, d_H, T, in_pitch,
                  d_taps, K, reinterpret_cast<float2 *>(d_out), out_pitch, p.nseg, vec);
     count_launches(1);
     BPGB_CUDA_TRY(cudaGetLastError());
