@@ -589,9 +589,13 @@ int bpgb_backproject_host(const void *transient_chunk, uint64_t transient_size, 
     };
     // A large capture is uploaded in parts, the pair splits of each part running while the
     // next one is copied (4,096 x 2,048 FP32 rows into 64^3 voxels: 588 -> 512 us).
-    const uint32_t parts = plan->fast && num_pairs * (size_t)T * esz >= (4u << 20)
-                               ? fast_plan_parts(plan->fast)
-                               : 1;
+    uint32_t parts = plan->fast ? fast_plan_parts(plan->fast) : 1;
+    if (!st && parts > 1) {
+        cudaPointerAttributes mem{};
+        if (cudaPointerGetAttributes(&mem, transient_chunk) != cudaSuccess) cudaGetLastError();
+        parts = host_parts(mem.type == cudaMemoryTypeHost, num_pairs * (uint64_t)T * esz,
+                           num_pairs * nvox, parts);
+    }
     thread_local HostStreams hs;
     if (!st && parts > 1 && hs.ready()) {
         // The call's streams don't order themselves after the legacy default stream, as a

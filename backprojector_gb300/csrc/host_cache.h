@@ -92,4 +92,18 @@ struct HostPlanCache {
     ~HostPlanCache() { clear(); }
 };
 
+// Parts (of at most `most`) in which a host call uploads its rows, the pair splits of each running
+// while the next one is copied.  Hidden is the shorter of upload (170 GB/s) and pass (3.6 x 10^12
+// updates/s), less the last part of it; each further copy and launch costs, from pageable memory about
+// 45 us in all, from pinned 10.  Measured at 2 to 128 MB into 8^3 to 96^3 voxels, single copy / four
+// parts in us: pageable 4 MB 32^3 105 / 144, 8 MB 64^3 421 / 420, 16 MB 32^3 211 / 224,
+// 48^3 307 / 254, 32 MB 64^3 577 / 506, 64 MB 40^3 588 / 600, 48^3 624 / 571; pinned 8 MB 16^3
+// 116 / 125, 48^3 244 / 241, 32 MB 32^3 275 / 263, 64^3 538 / 458.  From 2 x 10^9 updates on the cost
+// is under 1%.
+inline uint32_t host_parts(bool pinned, uint64_t bytes, uint64_t updates, uint32_t most) {
+    const bool hides = pinned ? bytes >= 8000000 && updates >= 100000000
+                              : bytes >= 11000000 && updates >= 300000000;
+    return hides || (bytes >= 4000000 && updates >= 2000000000) ? most : 1;
+}
+
 }  // namespace bpgb

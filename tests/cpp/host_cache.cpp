@@ -1,5 +1,6 @@
 // The per-thread caches of the host-buffer calls (host_cache.h) against a fake CUDA runtime of two
-// devices: a buffer or plan made on one device is never handed out on the other.  Exit status 0
+// devices: a buffer or plan made on one device is never handed out on the other; and when a capture
+// is uploaded in parts.  Exit status 0
 // when every check holds; the line of the first that fails otherwise.
 #include <cstdlib>
 #include <map>
@@ -54,5 +55,20 @@ int main() {
     CHECK(cache.find(0, pairs, 2, 9, n, nullptr, nullptr, 1.0f, 0.5f, o) == nullptr);
     cache.clear();
     CHECK(plans_destroyed == 1);
+
+    // One copy where parts hide less than they cost, measured at these bytes and updates; at most
+    // the parts that a plan has.
+    const uint64_t mb = 1 << 20;
+    CHECK(host_parts(false, 4 * mb, 1024ull * 32 * 32 * 32, 4) == 1);
+    CHECK(host_parts(true, 4 * mb, 1024ull * 32 * 32 * 32, 4) == 1);
+    CHECK(host_parts(false, 128 * mb, 16384ull * 8 * 8 * 8, 4) == 1);
+    CHECK(host_parts(true, 128 * mb, 16384ull * 8 * 8 * 8, 4) == 1);
+    CHECK(host_parts(false, 2 * mb, 576ull * 200 * 200 * 200, 4) == 1);
+    CHECK(host_parts(false, 32 * mb, 4096ull * 64 * 64 * 64, 4) == 4);
+    CHECK(host_parts(false, 32 * mb, 4096ull * 64 * 64 * 64, 2) == 2);
+    CHECK(host_parts(false, 32 * mb, 4096ull * 64 * 64 * 64, 1) == 1);
+    CHECK(host_parts(true, 32 * mb, 4096ull * 32 * 32 * 32, 4) == 4);
+    CHECK(host_parts(false, 32 * mb, 4096ull * 32 * 32 * 32, 4) == 1);
+    CHECK(host_parts(false, 8 * mb, 4096ull * 96 * 96 * 96, 4) == 4);
     return 0;
 }

@@ -1,5 +1,6 @@
-"""The host-buffer calls' per-thread caches belong to a device: tests/cpp/host_cache.cpp runs them
-against a fake CUDA runtime of two devices (no GPU)."""
+"""The host-buffer calls' per-thread caches belong to a device, and a capture is uploaded in parts only
+where that hides more than it costs: tests/cpp/host_cache.cpp runs both against a fake CUDA
+runtime of two devices (no GPU)."""
 from __future__ import annotations
 
 import subprocess
