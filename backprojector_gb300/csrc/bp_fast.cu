@@ -312,6 +312,14 @@ __device__ __forceinline__ uint2 bin_addresses(float2 y, uint32_t esz, float2 ba
     const float2 t = __ffma2_rn(n, make_float2((float)esz, (float)esz), base);
     return make_uint2(__float_as_uint(t.x), __float_as_uint(t.y));
 }
+// CHECKED: an address outside the `bytes` staged from `row` is counted and moved to the window's
+// first or last element.  (Addresses below 0 are negative floats, and NaN or huge positions large
+// ones, as integers too.)
+__device__ __forceinline__ uint32_t checked_address(uint32_t at, uint32_t row, uint32_t bytes,
+                                                    uint32_t esz, uint32_t &violations) {
+    violations += at - row >= bytes;
+    return (uint32_t)min(max((int32_t)at, (int32_t)row), (int32_t)(row + bytes - esz));
+}
 __device__ __forceinline__ float2 address_pair(uint32_t a) {
     return make_float2(__uint_as_float(a), __uint_as_float(a));
 }
@@ -329,7 +337,7 @@ struct Pair;
 
 template <>
 struct Pair<float> {
-    static constexpr uint32_t kEsz = 4, kShift = 2;
+    static constexpr uint32_t kEsz = 4;
     static constexpr bool kCplx = false;
     float2 a;
     __device__ __forceinline__ void zero() { a = make_float2(0.0f, 0.0f); }
@@ -352,7 +360,7 @@ struct Pair<float> {
 
 template <int IS_BF16>
 struct PairHalf {
-    static constexpr uint32_t kEsz = 2, kShift = 1;
+    static constexpr uint32_t kEsz = 2;
     static constexpr bool kCplx = false;
     float2 a;
     __device__ __forceinline__ void zero() { a = make_float2(0.0f, 0.0f); }
@@ -385,7 +393,7 @@ struct Pair<__nv_bfloat16> : PairHalf<1> {};
 
 template <>
 struct Pair<float2> {
-    static constexpr uint32_t kEsz = 8, kShift = 3;
+    static constexpr uint32_t kEsz = 8;
     static constexpr bool kCplx = true;
     float2 a0, a1;
     __device__ __forceinline__ void zero() { a0 = a1 = make_float2(0.0f, 0.0f); }
@@ -416,7 +424,7 @@ struct Pair<float2> {
 // its FP32 accumulator with the mixed-precision add.
 template <>
 struct Pair<__half2> {
-    static constexpr uint32_t kEsz = 4, kShift = 2;
+    static constexpr uint32_t kEsz = 4;
     static constexpr bool kCplx = true;
     float2 a0, a1;
     __device__ __forceinline__ void zero() { a0 = a1 = make_float2(0.0f, 0.0f); }
@@ -774,7 +782,6 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
     }
     uint32_t cur_l = ~0u;
     uint32_t violations = 0;
-    const float2 magic2 = make_float2(kMagic, kMagic);
 
     uint32_t stage = (uint32_t)(step0 % a.stages);
     uint32_t phase = (uint32_t)(step0 / a.stages) & 1;
@@ -857,15 +864,10 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
                 }
                 const float2 r = make_float2(rsqrt_approx(q.x), rsqrt_approx(q.y));
                 const float2 y = __ffma2_rn(q, r, Ae);
-                uint2 at;
+                uint2 at = bin_addresses(y, esz, base2);
                 if (CHECKED) {
-                    const float2 z = __fadd2_rn(y, magic2);
-                    uint32_t b0 = __float_as_uint(z.x) - kMagicBits, b1 = __float_as_uint(z.y) - kMagicBits;
-                    if (b0 >= a.W) violations++, b0 = (int32_t)b0 < 0 ? 0u : a.W - 1;
-                    if (b1 >= a.W) violations++, b1 = (int32_t)b1 < 0 ? 0u : a.W - 1;
-                    at = make_uint2(rbase + (b0 << PairT::kShift), rbase + (b1 << PairT::kShift));
-                } else {
-                    at = bin_addresses(y, esz, base2);
+                    at.x = checked_address(at.x, rbase, a.row_bytes, esz, violations);
+                    at.y = checked_address(at.y, rbase, a.row_bytes, esz, violations);
                 }
                 if (KAHAN)
                     part[p].gather2(at.x, at.y);
@@ -1114,7 +1116,6 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
     float2 B[kFactS][NP];
     uint32_t cur_sb = ~0u;
     uint32_t violations = 0;
-    const float2 magic2 = make_float2(kMagic, kMagic);
 
     uint32_t stage = (uint32_t)(step0 % a.stages);
     uint32_t phase = (uint32_t)(step0 / a.stages) & 1;
@@ -1155,16 +1156,12 @@ __device__ __forceinline__ bool fact_unit(const FastArgs &a, const CUtensorMap *
 #pragma unroll
                 for (int p = 0; p < NP; p++) {
                     const float2 y = __fadd2_rn(A[p], B[si][p]);
+                    uint2 at = bin_addresses(y, esz, base2);
                     if (CHECKED) {
-                        const float2 z = __fadd2_rn(y, magic2);
-                        uint32_t b0 = __float_as_uint(z.x) - kMagicBits, b1 = __float_as_uint(z.y) - kMagicBits;
-                        if (b0 >= a.W) violations++, b0 = (int32_t)b0 < 0 ? 0u : a.W - 1;
-                        if (b1 >= a.W) violations++, b1 = (int32_t)b1 < 0 ? 0u : a.W - 1;
-                        acc[p].gather2(rbase + (b0 << PairT::kShift), rbase + (b1 << PairT::kShift));
-                    } else {
-                        const uint2 at = bin_addresses(y, esz, base2);
-                        acc[p].gather2(at.x, at.y);
+                        at.x = checked_address(at.x, rbase, a.row_bytes, esz, violations);
+                        at.y = checked_address(at.y, rbase, a.row_bytes, esz, violations);
                     }
+                    acc[p].gather2(at.x, at.y);
                 }
             };
 #pragma unroll
