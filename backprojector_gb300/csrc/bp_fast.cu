@@ -2495,17 +2495,21 @@ struct BatchUnit {
 // The packed rows' tensor maps, one per box width of 128, 256 .. 1024 bytes (at most 256
 // elements): a capture's windows arrive in as few TMA boxes as a plan's would.
 constexpr uint32_t kBatchMaps = 8;
-constexpr uint32_t kBatchS = fact_spads(FACT_HALF);  // the factored launch runs that form
 struct BatchMaps {
     CUtensorMap m[kBatchMaps];
 };
 
-// FACT: the launch over the batch's lasers x SPADs captures (factored legs); otherwise the
-// launch over the rest (per-pair legs).  Each is one persistent launch over its own
-// cost-sorted unit list with its own counters; a batch with both kinds runs the two
-// launches back to back.
-template <typename HT, bool CHECKED, bool PLANAR, bool FACT>
-__global__ void __launch_bounds__(288, FACT ? fact_ctas(FACT_HALF) : 3)
+// The launches of a batch, by form: per-pair legs (FACT_NONE), and one for the lasers x SPADs captures
+// with factored legs, FACT_HALF or FACT_FULL.  Each is one persistent launch over its own
+// cost-sorted unit list with its own counters.
+constexpr int kForms = 3;
+__host__ __device__ constexpr uint32_t form_soft(int form) {  // bytes of a CTA's stages
+    return form == FACT_FULL ? 110 * 1024 : kWideSoft;
+}
+int form_of(const FastArgs &a) { return !a.fs ? FACT_NONE : a.halves == 2 ? FACT_HALF : FACT_FULL; }
+
+template <typename HT, bool CHECKED, bool PLANAR, int FORM>
+__global__ void __launch_bounds__(288, FORM == FACT_NONE ? 3 : fact_ctas(FORM))
     bp_batch_kernel(const __grid_constant__ BatchMaps maps, const BatchCap *__restrict__ caps,
                     const BatchUnit *__restrict__ units, uint32_t n_units,
                     const float4 *__restrict__ tables, float *__restrict__ out,
@@ -2544,10 +2548,13 @@ __global__ void __launch_bounds__(288, FACT ? fact_ctas(FACT_HALF) : 3)
         const CUtensorMap *tmap = &maps.m[cap_s.a.BW * Pair<HT>::kEsz / 128 - 1];
         // split captures write partial sums (reduced after the launch), the rest the volume
         float *dst = cap_s.a.splits > 1 ? scratch + cap_s.part_off : out + cap_s.out_off;
-        if constexpr (FACT)
-            ok = fact_unit<HT, CHECKED, FACT_HALF>(
+        if constexpr (FORM == FACT_HALF)
+            ok = fact_unit<HT, CHECKED, FORM>(
                 cap_s.a, tmap, tab, tab + cap_s.a.S, dst, diag, u.tile / 2, u.tile & 1, u.split,
                 (uint32_t)cap_s.row_base, step, sh);
+        else if constexpr (FORM == FACT_FULL)
+            ok = fact_unit<HT, CHECKED, FORM>(cap_s.a, tmap, tab, tab + cap_s.a.S, dst, diag, u.tile, 0,
+                                              u.split, (uint32_t)cap_s.row_base, step, sh);
         else
             ok = fast_unit<HT, 8, false, CHECKED, PLANAR, kBatchRows, false>(
                 cap_s.a, tmap, tab, tab + cap_s.a.S, dst, diag, u.tile, u.split,
@@ -2567,20 +2574,23 @@ __global__ void __launch_bounds__(288, FACT ? fact_ctas(FACT_HALF) : 3)
 }
 
 template <typename HT>
-void *batch_kernel_ptr(bool checked, bool planar, bool fact) {
-    if (fact)  // the planar-wall form is a per-pair body detail
-        return checked ? (void *)bp_batch_kernel<HT, true, false, true>
-                       : (void *)bp_batch_kernel<HT, false, false, true>;
+void *batch_kernel_ptr(bool checked, bool planar, int form) {
+    if (form == FACT_HALF)  // the planar-wall form is a per-pair body detail
+        return checked ? (void *)bp_batch_kernel<HT, true, false, FACT_HALF>
+                       : (void *)bp_batch_kernel<HT, false, false, FACT_HALF>;
+    if (form == FACT_FULL)
+        return checked ? (void *)bp_batch_kernel<HT, true, false, FACT_FULL>
+                       : (void *)bp_batch_kernel<HT, false, false, FACT_FULL>;
     if (planar)
-        return checked ? (void *)bp_batch_kernel<HT, true, true, false>
-                       : (void *)bp_batch_kernel<HT, false, true, false>;
-    return checked ? (void *)bp_batch_kernel<HT, true, false, false>
-                   : (void *)bp_batch_kernel<HT, false, false, false>;
+        return checked ? (void *)bp_batch_kernel<HT, true, true, FACT_NONE>
+                       : (void *)bp_batch_kernel<HT, false, true, FACT_NONE>;
+    return checked ? (void *)bp_batch_kernel<HT, true, false, FACT_NONE>
+                   : (void *)bp_batch_kernel<HT, false, false, FACT_NONE>;
 }
 
-void *select_batch_kernel(int dtype, bool checked, bool planar, bool fact) {
-    return dtype == BPGB_DTYPE_F16 ? batch_kernel_ptr<__half>(checked, planar, fact)
-                                   : batch_kernel_ptr<float>(checked, planar, fact);
+void *select_batch_kernel(int dtype, bool checked, bool planar, int form) {
+    return dtype == BPGB_DTYPE_F16 ? batch_kernel_ptr<__half>(checked, planar, form)
+                                   : batch_kernel_ptr<float>(checked, planar, form);
 }
 
 }  // namespace
@@ -2588,19 +2598,17 @@ void *select_batch_kernel(int dtype, bool checked, bool planar, bool fact) {
 struct BatchPlan {
     int dtype = BPGB_DTYPE_F32;
     bool checked = false, planar = false;
-    uint32_t n = 0, pitch = 0, stages = 0, chunk = 0, smem = 0, grid = 0, n_units = 0;
+    uint32_t n = 0, pitch = 0, n_units = 0;
     uint32_t boxes = 0;  // bit k: a capture stages boxes of (k + 1) x 128 bytes
-    // units [0, n_units - n_fact) run per-pair legs, the last n_fact factored legs (a
-    // second launch with grid_fact CTAs and the counters d_sched[2..3]); each launch has
-    // its own stage ring (ring[0] per-pair, ring[1] factored)
-    uint32_t n_fact = 0, grid_fact = 0;
+    // the launches by form: the units [unit0, unit0 + units), the counters d_sched[2 form] and
+    // d_sched[2 form + 1], and a stage ring each
     struct {
-        uint32_t chunk = 0, stages = 0, smem = 0;
-    } ring[2];
+        uint32_t chunk = 0, stages = 0, smem = 0, grid = 0, unit0 = 0, units = 0;
+    } launch[kForms];
     // captures whose units are split over pair ranges: partial sums in d_scratch, added
     // into the volume after their launch
     struct Split {
-        int fact;
+        int form;
         uint32_t splits;
         uint64_t part_off, out_off, nvox;
         float scale;
@@ -2614,7 +2622,7 @@ struct BatchPlan {
     BatchUnit *d_units = nullptr;
     float4 *d_tables = nullptr;
     unsigned long long *d_diag = nullptr;
-    unsigned int *d_sched = nullptr;  // work counter, finished-CTA counter
+    unsigned int *d_sched = nullptr;  // per form: work counter, finished-CTA counter
     cudaStream_t own_stream = nullptr;
     cudaStream_t side_stream = nullptr;  // the per-pair launch when both kinds run
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -2656,28 +2664,27 @@ int batch_execute(BatchPlan *b, const void *d_H, float *d_out, cudaStream_t s) {
     // stream forked from and joined back into `s` (two branches of a captured graph).
     // Their CTAs cannot share an SM (registers), so the per-pair CTAs take the SMs the
     // factored launch's last CTAs leave, and neither launch ends with an idle tail.
-    const uint32_t n_pp = b->n_units - b->n_fact;
-    const bool fork = n_pp && b->n_fact;
+    const bool fork = b->launch[FACT_NONE].units &&
+                      (b->launch[FACT_HALF].units || b->launch[FACT_FULL].units);
     if (fork) {
         BPGB_CUDA_TRY(cudaEventRecord(b->ev_fork, s));
         BPGB_CUDA_TRY(cudaStreamWaitEvent(b->side_stream, b->ev_fork, 0));
     }
-    for (int f = 1; f >= 0; f--) {
-        uint32_t nu = f ? b->n_fact : n_pp;
-        if (!nu) continue;
-        const cudaStream_t ls = (fork && f == 0) ? b->side_stream : s;
-        const BatchUnit *units = b->d_units + (f ? n_pp : 0);
-        unsigned int *sched = b->d_sched + (f ? 2 : 0);
-        void *kern = select_batch_kernel(b->dtype, b->checked, b->planar, f != 0);
+    for (int f = kForms - 1; f >= 0; f--) {
+        auto &l = b->launch[f];
+        if (!l.units) continue;
+        const cudaStream_t ls = (fork && f == FACT_NONE) ? b->side_stream : s;
+        const BatchUnit *units = b->d_units + l.unit0;
+        unsigned int *sched = b->d_sched + 2 * f;
+        void *kern = select_batch_kernel(b->dtype, b->checked, b->planar, f);
         void *args[] = {(void *)&map,         (void *)&b->d_caps,    (void *)&units,
-                        (void *)&nu,          (void *)&b->d_tables,  (void *)&d_out,
+                        (void *)&l.units,     (void *)&b->d_tables,  (void *)&d_out,
                         (void *)&b->d_scratch, (void *)&b->d_diag,   (void *)&sched,
-                        (void *)&b->ring[f].stages, (void *)&b->spin_limit};
-        BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3(f ? b->grid_fact : b->grid), dim3(288), args,
-                                       b->ring[f].smem, ls));
+                        (void *)&l.stages, (void *)&b->spin_limit};
+        BPGB_CUDA_TRY(cudaLaunchKernel(kern, dim3(l.grid), dim3(288), args, l.smem, ls));
         count_launches(1);
         for (const auto &sp : b->splits) {  // partial sums of this launch's split captures
-            if (sp.fact != f) continue;
+            if (sp.form != f) continue;
             launch_reduce_splits(b->d_scratch + sp.part_off, d_out + sp.out_off, sp.nvox, sp.splits,
                                  sp.scale, false, ls);
         }
@@ -2759,15 +2766,15 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         const bool confocal = fz.geom == GEOM_CONFOCAL;
         const uint64_t L = confocal ? 1 : fz.L;
         FastArgs &a = hc[c].a;
-        bool fact = fz.geom == GEOM_EXHAUSTIVE && !o.unfactored && fz.S % 4 == 0;
-        for (;;) {  // the per-pair form where the factored one does not fit
-            st = fast_args(a, cfg, vol, hd, confocal, g.deltaT, g.t0, L, fz.S, g.T, esz, false,
-                           o.chunk > 0 ? (uint32_t)o.chunk : 0,
-                           o.stages > 0 ? (uint32_t)o.stages : 0, &why,
-                           fact ? FACT_HALF : FACT_NONE);
-            if (!st || !fact) break;
-            fact = false;
-        }
+        const bool fact = fz.geom == GEOM_EXHAUSTIVE && !o.unfactored && fz.S % 4 == 0;
+        auto args = [&](int form) {
+            return fast_args(a, cfg, vol, hd, confocal, g.deltaT, g.t0, L, fz.S, g.T, esz, false,
+                             o.chunk > 0 ? (uint32_t)o.chunk : 0,
+                             o.stages > 0 ? (uint32_t)o.stages : 0, &why, form);
+        };
+        st = args(fact ? FACT_HALF : FACT_NONE);
+        if (fact && (st || a.chunk < 32)) st = args(FACT_FULL);  // few rows fit a stage
+        if (fact && st) st = args(FACT_NONE);  // nor a whole block of SPADs
         if (st) return fail(st, why);
         a.out_scale = g.h_scale != 0.0f ? g.h_scale : 1.0f;
         a.splits = 1;
@@ -2827,36 +2834,56 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         }
         planar = tdiag[2] == 0;
     }
+    // The factored captures run in one form, because launches of two forms take turns on the SMs:
+    // FACT_FULL when captures whose windows ask for it, as a plan's would, hold an eighth of the
+    // work.  Four captures of 20,736 pairs into 48^3 voxels, FP32 rows (half / full tiles): 4,096
+    // bins 5.04 / 2.53 ms, 2,048 bins 2.39 / 2.11, 512 bins 1.74 / 1.91; one of 4,096 bins with a sixth
+    // of the work among three narrow ones 1.32 / 1.13 (each in its own form 1.22), FP16 rows
+    // 1.11 / 1.04 (1.14).
+    double factored[kForms] = {};
+    for (const BatchCap &h : hc)
+        factored[form_of(h.a)] += (double)h.a.L * h.a.S * h.a.nvox;
+    const bool full = 7.0 * factored[FACT_FULL] >= factored[FACT_HALF];
+    for (BatchCap &h : hc)
+        if (h.a.fs) h.a.halves = full ? 1 : 2;
     // One stage ring per launch: the widest window among that launch's captures sets its
-    // row slot.  Both launches target three CTAs per SM (72 KB of shared memory
-    // each); factored captures need whole 4-SPAD blocks per stage and run per pair (their wider windows serve that form too) when their ring
-    // cannot hold them.
+    // row slot.  Factored captures need whole SPAD blocks per stage and run per pair (their wider
+    // windows serve that form too) when their ring cannot hold them.
+    auto blocks_of = [](int f, uint32_t ch) {  // rows of whole SPAD blocks
+        if (f == FACT_NONE) return ch;
+        const uint32_t fs = ch >= fact_spads(f) ? fact_spads(f) : 4;
+        return ch / fs * fs;
+    };
     auto ring_of = [&](int f, uint32_t row_bytes, uint32_t *chunk_out, uint32_t *stages_out) {
         uint32_t chunk = o.chunk > 0 ? std::min<uint32_t>((uint32_t)o.chunk, kMaxChunk) : cfg.chunk;
         uint32_t stages = o.stages > 0 ? std::min<uint32_t>((uint32_t)o.stages, 8) : cfg.stages;
         stages = std::max<uint32_t>(stages, 2);
-        const uint32_t soft = kWideSoft;
+        const uint32_t soft = form_soft(f);
         auto sb = [&](uint32_t ch) { return table_bytes_of(ch) + ch * row_bytes; };
         if (o.stages <= 0)
             while (stages > 2 && stages * sb(chunk) > soft) stages--;
         if (o.chunk <= 0)
             while (chunk > 4 && stages * sb(chunk) > soft) chunk = fewer_rows(chunk);
         while (chunk > 1 && stages * sb(chunk) > 200 * 1024) chunk = (chunk + 1) / 2;
-        if (f) chunk = chunk >= kBatchS ? chunk / kBatchS * kBatchS : chunk / 4 * 4;
+        chunk = blocks_of(f, chunk);
         *chunk_out = chunk;
         *stages_out = stages;
         return chunk > 0 && stages * sb(chunk) <= 200 * 1024;
     };
-    uint32_t row_bytes[2] = {0, 0};
-    for (uint32_t c = 0; c < n; c++)
-        row_bytes[hc[c].a.fs ? 1 : 0] = std::max(row_bytes[hc[c].a.fs ? 1 : 0], hc[c].a.row_bytes);
-    uint32_t chunk[2] = {0, 0}, stages[2] = {0, 0};
-    if (row_bytes[1] && !ring_of(1, row_bytes[1], &chunk[1], &stages[1])) {
-        for (uint32_t c = 0; c < n; c++) hc[c].a.fs = 0, hc[c].a.halves = 1;
-        row_bytes[0] = std::max(row_bytes[0], row_bytes[1]);
-        row_bytes[1] = 0;
+    uint32_t row_bytes[kForms] = {}, chunk[kForms] = {}, stages[kForms] = {};
+    for (uint32_t c = 0; c < n; c++) {
+        uint32_t &r = row_bytes[form_of(hc[c].a)];
+        r = std::max(r, hc[c].a.row_bytes);
     }
-    if (row_bytes[0] && !ring_of(0, row_bytes[0], &chunk[0], &stages[0])) {
+    for (int f : {FACT_HALF, FACT_FULL})
+        if (row_bytes[f] && !ring_of(f, row_bytes[f], &chunk[f], &stages[f])) {
+            for (uint32_t c = 0; c < n; c++)
+                if (form_of(hc[c].a) == f) hc[c].a.fs = 0, hc[c].a.halves = 1;
+            row_bytes[FACT_NONE] = std::max(row_bytes[FACT_NONE], row_bytes[f]);
+            row_bytes[f] = 0;
+        }
+    if (row_bytes[FACT_NONE] &&
+        !ring_of(FACT_NONE, row_bytes[FACT_NONE], &chunk[FACT_NONE], &stages[FACT_NONE])) {
         batch_free(b);
         return set_error(BPGB_ERR_UNSUPPORTED, "widest time window does not fit in shared memory");
     }
@@ -2864,30 +2891,27 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
     // windows take as many rows per stage as fit there (up to the preset's), unless the caller
     // fixed the rows.  With the wider boxes, 24-capture batch
     // 43.6 -> 40.1 ms.
-    uint32_t stage_bytes[2] = {0, 0};
-    for (int f = 0; f < 2; f++) {
+    uint32_t stage_bytes[kForms] = {};
+    for (int f = 0; f < kForms; f++) {
         if (!row_bytes[f]) continue;
         stage_bytes[f] = table_bytes_of(chunk[f]) + chunk[f] * row_bytes[f];
         if (o.chunk <= 0)
-            stage_bytes[f] = std::max<uint32_t>(stage_bytes[f], kWideSoft / stages[f] / 128 * 128);
-        b->ring[f].chunk = chunk[f];
-        b->ring[f].stages = stages[f];
-        b->ring[f].smem = stages[f] * stage_bytes[f] + 128;
+            stage_bytes[f] = std::max<uint32_t>(stage_bytes[f], form_soft(f) / stages[f] / 128 * 128);
+        b->launch[f].chunk = chunk[f];
+        b->launch[f].stages = stages[f];
+        b->launch[f].smem = stages[f] * stage_bytes[f] + 128;
     }
-    const int shown = row_bytes[0] ? 0 : 1;  // the ring bpgb_batch_info reports
-    b->chunk = chunk[shown];
-    b->stages = stages[shown];
-    b->smem = b->ring[shown].smem;
     b->planar = planar;
     b->pitch = (tmax + bw - 1) / bw * bw;
     for (uint32_t c = 0; c < n; c++) {
         FastArgs &a = hc[c].a;
-        const int f = a.fs ? 1 : 0;
+        const int f = form_of(a);
         uint32_t ch = chunk[f];
         if (o.chunk <= 0)
             while (ch + 4 <= cfg.chunk && table_bytes_of(ch + 4) + (ch + 4) * a.row_bytes <= stage_bytes[f])
                 ch += 4;
-        if (f) a.fs = ch >= kBatchS ? kBatchS : 4, ch = ch / a.fs * a.fs;
+        ch = blocks_of(f, ch);
+        if (f) a.fs = ch >= fact_spads(f) ? fact_spads(f) : 4;
         a.chunk = ch;
         a.stages = stages[f];
         a.table_bytes = table_bytes_of(ch);
@@ -2902,16 +2926,16 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
     }
     // resident CTAs of each launch
     cudaError_t e = cudaSuccess;
-    uint64_t resident[2] = {0, 0};
-    for (int f = 0; f < 2; f++) {
+    uint64_t resident[kForms] = {};
+    for (int f = 0; f < kForms; f++) {
         if (!row_bytes[f]) continue;
-        void *kern = select_batch_kernel(b->dtype, b->checked, b->planar, f != 0);
-        if (int rs = reserve_dynamic_smem(kern, b->ring[f].smem)) {
+        void *kern = select_batch_kernel(b->dtype, b->checked, b->planar, f);
+        if (int rs = reserve_dynamic_smem(kern, b->launch[f].smem)) {
             batch_free(b);
             return rs;
         }
         int occ = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 288, b->ring[f].smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 288, b->launch[f].smem);
         if (e != cudaSuccess || occ < 1) {
             batch_free(b);
             return e != cudaSuccess ? cuda_error(e, "batch kernel attributes")
@@ -2927,18 +2951,18 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         const FastArgs &a = hc[c].a;
         return (double)a.L * a.S * a.tdim[0] * a.tdim[1] * a.tdim[2] / a.halves;
     };
-    double share[2] = {0.0, 0.0};
+    double share[kForms] = {};
     for (uint32_t c = 0; c < n; c++) {
         const FastArgs &a = hc[c].a;
-        share[a.fs ? 1 : 0] += unit_cost(c) * a.halves * a.tiles[0] * a.tiles[1] * a.tiles[2];
+        share[form_of(a)] += unit_cost(c) * a.halves * a.tiles[0] * a.tiles[1] * a.tiles[2];
     }
-    for (int f = 0; f < 2; f++)
+    for (int f = 0; f < kForms; f++)
         if (resident[f]) share[f] /= (double)resident[f];
     uint64_t scratch = 0;
     std::vector<BatchUnit> units;
     for (uint32_t c = 0; c < n; c++) {
         FastArgs &a = hc[c].a;
-        const int f = a.fs ? 1 : 0;
+        const int f = form_of(a);
         const double target = share[f] / 24.0;  // unit length aimed at
         uint64_t sp = target > 0.0 ? (uint64_t)std::llround(unit_cost(c) / target) : 1;
         sp = std::max<uint64_t>(1, std::min<uint64_t>({sp, 8, fast_items(a)}));
@@ -2949,18 +2973,18 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
             b->splits.push_back({f, (uint32_t)sp, scratch, hc[c].out_off, a.nvox, a.out_scale});
             scratch += sp * a.nvox;
         }
-        // units' tile field: half tiles (2 x tile + half) in the factored launch
+        // units' tile field: 2 x tile + half in the launch of half tiles
         const uint64_t ntiles = (uint64_t)a.tiles[0] * a.tiles[1] * a.tiles[2] * a.halves;
         for (uint32_t k = 0; k < sp; k++)
             for (uint64_t t = 0; t < ntiles; t++) units.push_back({c, (uint32_t)t, k});
     }
-    // per-pair units first, then the factored ones; each list longest first
+    // a list per form; each longest first
     std::vector<uint32_t> order(units.size());
     for (uint32_t i = 0; i < order.size(); i++) order[i] = i;
     auto cost_of = [&](const BatchUnit &u) { return unit_cost(u.cap) / hc[u.cap].a.splits; };
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-        const bool fx = hc[units[x].cap].a.fs != 0, fy = hc[units[y].cap].a.fs != 0;
-        if (fx != fy) return fy;
+        const int fx = form_of(hc[units[x].cap].a), fy = form_of(hc[units[y].cap].a);
+        if (fx != fy) return fx < fy;
         return cost_of(units[x]) > cost_of(units[y]);
     });
     std::vector<BatchUnit> sorted(units.size());
@@ -2970,17 +2994,20 @@ int bpgb_batch_create(bpgb_batch *out, const bpgb_capture_geometry *caps, uint32
         return set_error(BPGB_ERR_UNSUPPORTED, "too many work units");
     }
     b->n_units = (uint32_t)sorted.size();
-    for (const BatchUnit &u : sorted) b->n_fact += hc[u.cap].a.fs ? 1 : 0;
-    b->grid = (uint32_t)std::min<uint64_t>(b->n_units - b->n_fact, resident[0]);
-    b->grid_fact = (uint32_t)std::min<uint64_t>(b->n_fact, resident[1]);
+    for (const BatchUnit &u : sorted) b->launch[form_of(hc[u.cap].a)].units++;
+    for (int f = 0; f < kForms; f++) {
+        auto &l = b->launch[f];
+        if (f) l.unit0 = b->launch[f - 1].unit0 + b->launch[f - 1].units;
+        l.grid = (uint32_t)std::min<uint64_t>(l.units, resident[f]);
+    }
     if (scratch) e = cudaMalloc(&b->d_scratch, scratch * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_caps, n * sizeof(BatchCap));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_units, sorted.size() * sizeof(BatchUnit));
     if (e == cudaSuccess) e = cudaMemcpy(b->d_caps, hc.data(), n * sizeof(BatchCap), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(b->d_units, sorted.data(), sorted.size() * sizeof(BatchUnit), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_sched, 4 * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMemset(b->d_sched, 0, 4 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_sched, 2 * kForms * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMemset(b->d_sched, 0, 2 * kForms * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
@@ -3010,10 +3037,13 @@ int bpgb_batch_get_info(bpgb_batch b, bpgb_batch_info *info) {
     info->total_rows = b->total_rows;
     info->total_voxels = b->total_vox;
     info->work_units = b->n_units;
-    info->grid = std::max(b->grid, b->grid_fact);
-    info->stages = b->stages;
-    info->chunk = b->chunk;
-    info->smem_bytes = b->smem;
+    // of the per-pair launch where there is one
+    int shown = FACT_NONE;
+    while (shown + 1 < kForms && !b->launch[shown].units) shown++;
+    info->stages = b->launch[shown].stages;
+    info->chunk = b->launch[shown].chunk;
+    info->smem_bytes = b->launch[shown].smem;
+    for (const auto &l : b->launch) info->grid = std::max(info->grid, l.grid);
     info->updates = b->updates;
     info->planar = b->planar ? 1 : 0;
     return BPGB_OK;
