@@ -7,8 +7,9 @@
 // and H[p, b] is added when 0 <= b <= T-1 (:157-159).  The arithmetic below is the same
 // expression in the same order (FMA-contracted voxel position, norm3df, IEEE division,
 // round-half-away), so every bin index equals the reference's; only the summation order
-// differs (register sums in pair order instead of strided partial sums plus a serial
-// shared-memory reduction).  This file must be compiled without fast-math flags.
+// differs (register sums of a group's updates in pair order, then its marked updates, then the
+// pair splits, instead of strided partial sums plus a serial shared-memory reduction).  This file
+// must be compiled without fast-math flags.
 //
 // Evaluating that expression costs about 100 instructions per update (two norm3df, an
 // IEEE divide, roundf), and the reference's result is needed to the last bit only where the
@@ -19,10 +20,12 @@
 // reference's bin; the other updates (about 2 E of them) are marked in a bit mask per
 // thread and evaluated with the reference's expression after each group of 64 pairs, one
 // marked pair per lane at a time, so that a warp spends one evaluation on the marks of all
-// its lanes.  E = 0.5 (scales where the bound does not hold) marks every update.
+// its lanes.  Where E is no use (scales where the bound does not hold, E = 0.5, or small launches that
+// would wait for their marks) a direct kernel evaluates the expression for every update.
 //
 // Bound: issue (24 to 28 instructions per update, the marked ones' evaluations included) and the
-// latency of the L1 gathers.  Measured on 64 x 64 pairs that do not factor, T = 2048, 64^3
+// latency of the L1 gathers, at 70 or 72 registers and so 13 or 14 CTAs per SM (complex rows with
+// range checks spill 16 bytes).  Measured on 64 x 64 pairs that do not factor, T = 2048, 64^3
 // voxels: 3.60 ms before, 0.95 ms with the filter.
 //
 // Layout: one CTA = 64 threads = a 4 x 4 x 16 voxel tile (z fastest, x slowest), the four

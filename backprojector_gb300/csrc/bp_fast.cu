@@ -518,9 +518,10 @@ __device__ __forceinline__ uint32_t group_origin(const FastArgs &a, uint32_t &sp
 }
 
 // The consumer side of `count` steps for a warp whose whole sub-block lies past the volume's
-// edge (a tile's x or z overhang): it only releases the stages.  101 voxels along z leave 2 of
-// 28 warp columns idle: 90 x 75 x 101 voxels 924 -> 879 us.  (Skipping the rows by a flag in
-// the consumers' own loop cost every volume 5-8% instead.)
+// edge (a tile's x or z overhang): it only releases the stages.  A warp of the default tile covers
+// 4 x 8 x 8 voxels, so 90 x 75 x 101 voxels leave 1 of 24 warp columns along x and 1 of 14 along z
+// idle (924 -> 879 us with the 8 x 8 x 4 warps of the time, whose columns left 2 of 28 along z).
+// (Skipping the rows by a flag in the consumers' own loop cost every volume 5-8% instead.)
 __device__ __forceinline__ bool release_stages(const FastArgs &a, const PipeShared &sh,
                                                unsigned long long *diag, uint64_t step0,
                                                uint32_t count) {
@@ -832,8 +833,8 @@ __device__ __forceinline__ bool fast_unit(const FastArgs &a, const CUtensorMap *
             for (int p = 0; p < NP; p++) part[p].zero();
         }
         // ROWS rows per unrolled iteration give the scheduler ROWS x NP independent
-        // voxel-pair chains to interleave (one row for complex rows, whose accumulators
-        // already double the registers).  Measured: 256^3 voxels 4 rows
+        // voxel-pair chains to interleave (two rows for complex64 and four for FP16 pairs, whose
+        // accumulators already double the registers).  Measured: 256^3 voxels 4 rows
         // 75.4 ms, 8 rows 73.6, 16 rows 69.6; four 8^3 tiles per CTA (learned octree) 4 rows
         // 3.47 ms, 8 rows 3.32, 16 rows 3.38; the batch kernel 4 rows 36.96, 8 rows 36.74, 16 rows
         // 36.91; complex64 rows (128^3) 1 row 16.14, 2 rows 16.08.
@@ -2474,8 +2475,7 @@ void fast_plan_free(FastPlan *fp) {
 // Batches: many captures of uneven grids, T and volumes in persistent launches.
 //
 // All captures' rows live in one packed device buffer [sum P_c, pitch] (capture c at
-// rows row_base_c; bins T_c..pitch zero) behind a single TMA tensor map whose box width
-// is shared.  Each capture has a launch descriptor (FastArgs, table, output and partial-sum
+// rows row_base_c; bins T_c..pitch zero) behind a TMA tensor map per box width.  Each capture has a launch descriptor (FastArgs, table, output and partial-sum
 // offsets) in device memory.  The work lists hold (capture, tile, pair range) units, one
 // list per launch (per-pair legs; factored lasers x SPADs legs), each sorted by cost
 // (pairs x tile voxels / ranges) in decreasing order; each CTA takes the next unit from

@@ -90,8 +90,9 @@ typedef struct bpgb_options {
                             block-sparse passes, 13: four 8^3 tiles per CTA (real rows,
                             plain sums) */
     int32_t pair_splits; /* CTAs sharing one voxel tile over disjoint pair ranges (0 = auto,
-                            negative = plans: as many as fill two rounds of CTAs, so that sums
-                            do not move with the automatic choice) */
+                            negative = plans: a division of the sums that does not move with
+                            the automatic choices -- as many splits as fill two rounds of CTAs,
+                            over stages of the preset's rows halved until they fit 72 KB) */
     int32_t checked;     /* 1 = clamp and count out-of-window bins (tests) */
     uint32_t spin_limit; /* bounded mbarrier waits: polls before giving up (0 = default) */
     int32_t chunk;       /* FAST: SPAD rows per pipeline stage, 1..64 (0 = from the preset;
