@@ -41,43 +41,39 @@ unsigned blocks_for(const Rows &g) {
     return (unsigned)(n < kSms * 16 ? n : kSms * 16);
 }
 
-// Padded rows too short to occupy a CTA each share one: `lanes` threads per row, up to four
-// elements each, and four rows of a thread in flight.  A CTA per row took 121 us for the
-// largest of 200,000 rows of 8 elements and 116 us for their conversion, against 12.3 and 8.2 us with
-// one element and a division per thread; 6.2 and 5.9 us now.
+// Padded rows too short to occupy a CTA each: a CTA takes `share` of them at a time as one run of
+// share x width elements, whose row and place a multiplication with 2^32 / width gives (exact
+// below 2^32 / width elements).  A CTA per row took 121 us for the largest of 200,000 rows of 8
+// elements and 116 us for their conversion, against 12.3 and 8.2 us with one element and a
+// 64-bit division per thread; 6.5 and 5.0 us now.
 constexpr uint32_t kShortRow = 512;
-constexpr uint32_t kRowsInFlight = 4;
 
 struct ShortRows {
-    uint64_t rows;
-    uint32_t T, pitch, lanes;  // a power of two
-
-    uint64_t units() const {  // of kRowsInFlight rows per thread
-        const uint64_t per = kRowsInFlight * (256 / lanes);
-        return (rows + per - 1) / per;
-    }
+    uint64_t rows, units;
+    uint32_t width, share, inverse;
 };
 
-ShortRows short_rows(uint64_t rows, uint32_t T, uint32_t pitch, uint32_t width) {
-    ShortRows g{rows, T, pitch, 1};
-    while (g.lanes < 256 && g.lanes < width) g.lanes *= 2;
-    // fewer threads per row, down to a warp, where the rows still make eight CTAs per SM
-    while (g.lanes > 32 && 2 * g.lanes >= width) {
-        ShortRows h = g;
-        h.lanes /= 2;
-        if (h.units() < 8 * kSms) break;
-        g = h;
-    }
-    return g;
+ShortRows short_rows(uint64_t rows, uint32_t width) {
+    // 4,096 elements a unit, fewer until every SM has eight units
+    uint32_t elements = 4096;
+    while (elements > 512 && rows * width < (uint64_t)elements * 8 * kSms) elements /= 2;
+    const uint32_t share = elements > width ? elements / width : 1;
+    return {rows, (rows + share - 1) / share, width, share, (uint32_t)((1ull << 32) / width + 1)};
 }
 
 unsigned blocks_for(const ShortRows &g) {
-    const uint64_t n = g.units();
-    return (unsigned)(n < kSms * 16 ? n : kSms * 16);
+    return (unsigned)(g.units < kSms * 16 ? g.units : kSms * 16);
 }
 
-__device__ __forceinline__ uint64_t short_row(const ShortRows &g, uint64_t unit, uint32_t k) {
-    return (unit * kRowsInFlight + k) * (256 / g.lanes) + threadIdx.x / g.lanes;
+// f(row from the unit's first, place, element of the unit) for this thread's elements of unit q.
+template <typename F>
+__device__ __forceinline__ void short_elements(const ShortRows &g, uint64_t q, F &&f) {
+    const uint32_t n = (uint32_t)min((uint64_t)g.share, g.rows - q * g.share) * g.width;
+#pragma unroll 4
+    for (uint32_t e = threadIdx.x; e < n; e += 256) {
+        const uint32_t r = g.width == 1 ? e : __umulhi(e, g.inverse);
+        f(r, e - r * g.width, e);
+    }
 }
 
 // The CTA's largest |value| as float bits into out[0] (NaN counts as +inf).
@@ -93,23 +89,16 @@ __device__ __forceinline__ void block_max(unsigned int m, unsigned int *out) {
 }
 
 __global__ void __launch_bounds__(256)
-    absmax_short_kernel(const float *__restrict__ in, const ShortRows g, uint64_t units,
+    absmax_short_kernel(const float *__restrict__ in, const ShortRows g, uint32_t pitch,
                         unsigned int *__restrict__ out) {
     wait_previous();
     unsigned int m = 0;
-    for (uint64_t q = blockIdx.x; q < units; q += gridDim.x)
-#pragma unroll 2
-        for (uint32_t t = threadIdx.x & (g.lanes - 1); t < g.T; t += g.lanes) {
-            float v[kRowsInFlight];
-#pragma unroll
-            for (uint32_t k = 0; k < kRowsInFlight; k++) {
-                const uint64_t r = short_row(g, q, k);
-                v[k] = r < g.rows ? __ldg(in + r * g.pitch + t) : 0.0f;
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kRowsInFlight; k++)
-                m = max(m, __float_as_uint(v[k]) & 0x7fffffffu);
-        }
+    for (uint64_t q = blockIdx.x; q < g.units; q += gridDim.x) {
+        const float *src = in + q * g.share * pitch;
+        short_elements(g, q, [&](uint32_t r, uint32_t t, uint32_t) {
+            m = max(m, __float_as_uint(__ldg(src + (uint64_t)r * pitch + t)) & 0x7fffffffu);
+        });
+    }
     block_max(m, out);
 }
 
@@ -190,25 +179,18 @@ __global__ void __launch_bounds__(256)
 // The same for short padded rows.
 template <typename HT>
 __global__ void __launch_bounds__(256)
-    to_half_short_kernel(const float *__restrict__ in, const ShortRows g, uint64_t units,
-                         uint32_t out_pitch, float scale, const float *__restrict__ d_absmax,
-                         float target, HT *__restrict__ out) {
+    to_half_short_kernel(const float *__restrict__ in, const ShortRows g, uint32_t T, uint32_t pitch,
+                         float scale, const float *__restrict__ d_absmax, float target,
+                         HT *__restrict__ out) {
     wait_previous();
     const float inv_scale = 1.0f / scale_of(scale, d_absmax, target);
-    for (uint64_t q = blockIdx.x; q < units; q += gridDim.x)
-        for (uint32_t t = threadIdx.x & (g.lanes - 1); t < out_pitch; t += g.lanes) {
-            float v[kRowsInFlight];
-#pragma unroll
-            for (uint32_t k = 0; k < kRowsInFlight; k++) {
-                const uint64_t r = short_row(g, q, k);
-                v[k] = r < g.rows && t < g.T ? __ldg(in + r * g.pitch + t) * inv_scale : 0.0f;
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kRowsInFlight; k++) {
-                const uint64_t r = short_row(g, q, k);
-                if (r < g.rows) store_h(out + r * out_pitch + t, v[k]);
-            }
-        }
+    for (uint64_t q = blockIdx.x; q < g.units; q += gridDim.x) {
+        const float *src = in + q * g.share * pitch;
+        HT *dst = out + q * g.share * g.width;
+        short_elements(g, q, [&](uint32_t r, uint32_t t, uint32_t e) {
+            store_h(dst + e, t < T ? __ldg(src + (uint64_t)r * pitch + t) * inv_scale : 0.0f);
+        });
+    }
 }
 
 // out[r][t] = in[r][from + t] for 0 <= from + t < T, else 0 (t < out_pitch).
@@ -264,8 +246,8 @@ int bpgb_rows_absmax(const float *d_H, uint64_t rows, uint32_t T, uint32_t pitch
     const uint64_t n = rows * T;
     if (n == 0) return BPGB_OK;
     if (rows > 1 && pitch != T && T <= kShortRow) {
-        const ShortRows g = short_rows(rows, T, pitch, T);
-        launch_after(absmax_short_kernel, blocks_for(g), 256, 0, s, d_H, g, g.units(),
+        const ShortRows g = short_rows(rows, T);
+        launch_after(absmax_short_kernel, blocks_for(g), 256, 0, s, d_H, g, pitch,
                      (unsigned int *)d_max);
         count_launches(1);
         BPGB_CUDA_TRY(cudaGetLastError());
@@ -294,10 +276,10 @@ int bpgb_rows_to_half(const float *d_H, uint64_t rows, uint32_t T, uint32_t in_p
     cudaStream_t s = (cudaStream_t)stream;
     const bool flat = in_pitch == T && out_pitch == T;
     if (rows > 1 && !flat && out_pitch <= kShortRow) {
-        const ShortRows g = short_rows(rows, T, in_pitch, out_pitch);
+        const ShortRows g = short_rows(rows, out_pitch);
         auto run = [&](auto kernel, auto *out) {
-            launch_after(kernel, blocks_for(g), 256, 0, s, d_H, g, g.units(), out_pitch, scale, d_absmax,
-                         target, out);
+            launch_after(kernel, blocks_for(g), 256, 0, s, d_H, g, T, in_pitch, scale, d_absmax, target,
+                         out);
         };
         dtype == BPGB_DTYPE_F16 ? run(to_half_short_kernel<__half>, (__half *)d_out)
                                 : run(to_half_short_kernel<__nv_bfloat16>, (__nv_bfloat16 *)d_out);

@@ -10,8 +10,8 @@ from backprojector_gb300 import capi
 pytestmark = pytest.mark.gpu
 
 
-# rows that share a CTA (a thread to a warp each, four accesses per thread above), a CTA per row,
-# and few long rows in pieces of 1,024 to 16,384
+# rows that share a CTA (units of 512 to 4,096 elements, whole and cut), a CTA per row, and few long
+# rows in pieces of 1,024 to 16,384
 @pytest.mark.parametrize("rows,T,pitch,out_pitch", [
     (1000, 1, 2, 8), (777, 2, 3, 2), (1025, 3, 4, 4), (513, 8, 9, 9), (300, 31, 32, 32), (129, 33, 36, 40),
     (70, 127, 128, 128), (65, 129, 132, 136), (40, 512, 516, 512), (33, 1023, 1024, 1025),
